@@ -1,0 +1,53 @@
+// cg_loop.h — the resident minimizer loop (cg_loop.cu): one kernel that runs a
+// whole CGMethod::minimize on a team of thread blocks.
+#pragma once
+
+#include <vector>
+
+#include "handle.h"
+
+namespace mb {
+
+// What one team needs of its network; pointers into the handle's buffers.
+struct LoopArgs {
+    ChainDev ch;
+    DeviceFF ff;
+    int n3;            // coordinate components
+    int vb;            // blocks of the vector passes' summation order (vec_blocks, or 1)
+    int fixed;         // deterministic force sums
+    double *x, *d, *f0, *f1, *min_e;
+    CGState* st;       // parameters in, final state out
+    LambdaSet* lam;    // pending step sizes when the loop hands over
+    double* eout;      // [2][MEDYAN_FF_COUNT + 1]: energies before and after
+    double* erow;      // [2][kMaxLambda][4][loop_row_count]
+    double* vrow;      // [2][vb, or the 8 warps of a single one][4]: of the sums, of max|d|
+    int* words;        // kLoopWords words, zero at the launch
+    int* status;       // force status bits
+};
+
+// words: two pass flags (a pair needs a quadrature fallback), the loop's
+// outcome, the grid barrier's counter.
+constexpr int kLoopWords = 4;
+constexpr int kLoopThreads = 256;
+// words[2] at the end: the minimization is complete; it stopped in the loop
+// and the graph loop takes over from *st; it stopped in the setup, nothing is
+// changed but the force buffers; a grid barrier gave up.
+constexpr int kLoopDone = 0, kLoopHandOver = 1, kLoopRestart = 2, kLoopLost = 3;
+
+constexpr int kLoopCluster = 16;    // teams of up to this many blocks are thread-block clusters
+constexpr int kLoopGrid = 148;      // blocks of the largest team, a cooperative grid (one block per SM)
+constexpr int kLoopBeads = 250000;  // larger networks run in the graph loop
+
+// Blocks of a team for this network, 0 when the network is better off in the
+// graph loop.
+int loop_team(const ChainDev& ch, const DeviceFF& ff);
+// Energy rows of a pass at one step size, and the doubles that the rows and the
+// vector passes' sums take.
+int loop_row_count(const ChainDev& ch, const DeviceFF& ff);
+size_t loop_erow_doubles(int rows);
+__host__ __device__ __forceinline__ size_t loop_vrow_doubles(int vb) { return 2 * (size_t)(vb == 1 ? 8 : vb) * 4; }
+// Kernel attributes, per device; before the first launch.
+cudaError_t init_cg_loop();
+cudaError_t launch_cg_loop(const LoopArgs& a, int prec, int team, cudaStream_t s);
+
+}  // namespace mb

@@ -203,6 +203,12 @@ struct medyan_mech {
     mb::DevBuf<double> cg_dir, cg_force2, cg_min_coords, cg_part, cg_eout;
     mb::DevBuf<mb::CGState> cg_state;
     mb::DevBuf<mb::LambdaSet> cg_lam;
+    // resident loop (cg_loop.cu): partial rows, control words; the team of the
+    // minimization in flight (0: the graph loop)
+    mb::DevBuf<double> cg_rows;
+    mb::DevBuf<int> cg_words;
+    int cg_team = 0;
+    medyan_cg_params cg_params{};
     cudaGraphExec_t cg_graph = nullptr;   // instantiated minimization graph
     // pinned host staging of a minimization's inputs and results, so that
     // enqueueing it never waits on the device (batched minimization)
@@ -212,7 +218,9 @@ struct medyan_mech {
     // (energies, force status), so their copies are asynchronous
     struct SmallPinned {
         double energy[MEDYAN_FF_COUNT + 1];
+        double cg_energy[2 * (MEDYAN_FF_COUNT + 1)];
         int force_status;
+        int cg_words[4];
     }* small = nullptr;
     int cg_graph_prec = -1;
     long long cg_graph_gen = -1;          // ff_gen the graph was captured with

@@ -30,7 +30,7 @@
 // Built with --fmad=false (the excluded-volume formula and the quadrature
 // fallbacks round as the reference's code does).
 #include "handle.h"
-#include "potentials.cuh"
+#include "records.cuh"
 #include "excl.cuh"
 #include "quadrature.cuh"
 #include "pass.h"
@@ -93,9 +93,6 @@ namespace mb {
 namespace {
 
 constexpr int kSlots = MEDYAN_FF_COUNT;
-constexpr int kWarpOut = 30;  // forces written per warp tile: lanes 1..30 of 32 centres
-constexpr unsigned char kLink = 1, kBend = 2;
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kZeroThreads = 256;
 // Resident blocks of the main kernel per SM: 80 registers a thread, room
 // for a chain tile's loads in flight beside the one being computed
@@ -106,21 +103,6 @@ constexpr int main_blocks_per_sm() {
     return kMainBlocksPerSM;
 }
 constexpr int kExclThreadsMax = 128;
-
-__device__ __forceinline__ V3 shfl_up3(const V3& v) {
-    return V3{__shfl_up_sync(kFull, v.x, 1), __shfl_up_sync(kFull, v.y, 1), __shfl_up_sync(kFull, v.z, 1)};
-}
-__device__ __forceinline__ V3 shfl_down3(const V3& v) {
-    return V3{__shfl_down_sync(kFull, v.x, 1), __shfl_down_sync(kFull, v.y, 1), __shfl_down_sync(kFull, v.z, 1)};
-}
-template <class R>
-__device__ __forceinline__ T3<R> shfl_up3(const T3<R>& v) {
-    return T3<R>{__shfl_up_sync(kFull, v.x, 1), __shfl_up_sync(kFull, v.y, 1), __shfl_up_sync(kFull, v.z, 1)};
-}
-template <class R>
-__device__ __forceinline__ T3<R> shfl_down3(const T3<R>& v) {
-    return T3<R>{__shfl_down_sync(kFull, v.x, 1), __shfl_down_sync(kFull, v.y, 1), __shfl_down_sync(kFull, v.z, 1)};
-}
 
 // Positions of a pass: x, or x + lam*d rounded as calcCoordLineSearch.
 struct Pos {
@@ -403,95 +385,7 @@ __device__ __forceinline__ void chain_compute(const PassArgs& a, const Pos& P, d
     if (lane == 0) cprev = ce;
     if (lane == 31) cnext = ce;
     const bool own = lane >= 1 && lane <= kWarpOut && in;
-    if constexpr (F) {
-        T3<R> Fl{0, 0, 0}, A{0, 0, 0}, B{0, 0, 0};
-        if (fl & kLink) Fl = stretch_force<R>(c, cnext, r.lp.x, r.lp.y);
-        if (fl & kBend) bend_force<R>(diff<R>(cprev, c), diff<R>(c, cnext), r.bp.x, r.bp.y, A, B);
-        const T3<R> Fp = shfl_up3(Fl), Bp = shfl_up3(B), An = shfl_down3(A);
-        if (own) {
-            // link (q-1, q) acts on q; link (q, q+1) reacts on q; bends centred
-            // at q-1 (third bead), q (middle), q+1 (first bead); summed in double
-            const double fx = double(Fp.x) - double(Fl.x) + double(Bp.x) + (double(A.x) - double(B.x)) - double(An.x);
-            const double fy = double(Fp.y) - double(Fl.y) + double(Bp.y) + (double(A.y) - double(B.y)) - double(An.y);
-            const double fz = double(Fp.z) - double(Fl.z) + double(Bp.z) + (double(A.z) - double(B.z)) - double(An.z);
-            target_add(a.t, f, 3 * q, fx, fy, fz);
-        }
-    }
-    if constexpr (E) {
-        if (own) {
-            if (fl & kLink) acc[0] += stretch_energy<double>(c, cnext, r.lp.x, r.lp.y);
-            if (fl & kBend) acc[1] += bend_energy<double>(diff<double>(cprev, c), diff<double>(c, cnext), r.bp.x, r.bp.y);
-        }
-    }
-}
-
-// Record i of bonded segment s (0 leftover stretch, 1 leftover bend, 2
-// linker, 3 motor, 5 boundary): energy into acc[0], forces added to f.
-template <class R, bool E, bool F>
-__device__ __forceinline__ void bonded_record(const DeviceFF& ff, const ForceTarget& t, const Pos& P,
-                                              double* __restrict__ f, int s, int i, double (&acc)[4]) {
-    switch (s) {
-        case 0:
-            if (i < ff.n_stretch) {
-                const int2 q = ff.stretch_bs[i];
-                const double2 p = ff.stretch_p[i];
-                const V3 c1 = P(q.x), c2 = P(q.y);
-                if constexpr (E) acc[0] += stretch_energy<double>(c1, c2, p.x, p.y);
-                if constexpr (F) {
-                    const T3<R> Fs = stretch_force<R>(c1, c2, p.x, p.y);
-                    target_add(t, f, q.y, Fs.x, Fs.y, Fs.z);
-                    target_add(t, f, q.x, -Fs.x, -Fs.y, -Fs.z);
-                }
-            }
-            break;
-        case 1:
-            if (i < ff.n_bend) {
-                const int4 q = ff.bend_bs[i];
-                const double2 p = ff.bend_p[i];
-                const V3 c1 = P(q.x), c2 = P(q.y), c3 = P(q.z);
-                if constexpr (E) acc[0] += bend_energy<double>(diff<double>(c1, c2), diff<double>(c2, c3), p.x, p.y);
-                if constexpr (F) {
-                    T3<R> Fr1, Fr2;
-                    bend_force<R>(diff<R>(c1, c2), diff<R>(c2, c3), p.x, p.y, Fr1, Fr2);
-                    target_add(t, f, q.x, -Fr1.x, -Fr1.y, -Fr1.z);
-                    target_add(t, f, q.y, Fr1.x - Fr2.x, Fr1.y - Fr2.y, Fr1.z - Fr2.z);
-                    target_add(t, f, q.z, Fr2.x, Fr2.y, Fr2.z);
-                }
-            }
-            break;
-        case 2:
-        case 3: {
-            const int n = s == 2 ? ff.n_linker : ff.n_motor;
-            if (i < n) {
-                const int4 q = s == 2 ? ff.linker_bs[i] : ff.motor_bs[i];
-                const double4 p = s == 2 ? ff.linker_p[i] : ff.motor_p[i];
-                const V3 c1 = P(q.x), c2 = P(q.y), c3 = P(q.z), c4 = P(q.w);
-                if constexpr (E) acc[0] += spring_energy<double>(c1, c2, c3, c4, p.x, p.y, p.z, p.w);
-                if constexpr (F) {
-                    const T3<R> Fl = spring_force<R>(c1, c2, c3, c4, p.x, p.y, p.z, p.w);
-                    const R a1 = R(1) - R(p.z), a2 = R(p.z), b1 = R(1) - R(p.w), b2 = R(p.w);
-                    target_add(t, f, q.x, -Fl.x * a1, -Fl.y * a1, -Fl.z * a1);
-                    target_add(t, f, q.y, -Fl.x * a2, -Fl.y * a2, -Fl.z * a2);
-                    target_add(t, f, q.z, Fl.x * b1, Fl.y * b1, Fl.z * b1);
-                    target_add(t, f, q.w, Fl.x * b2, Fl.y * b2, Fl.z * b2);
-                }
-            }
-            break;
-        }
-        default:
-            if (i < ff.n_boundary) {
-                const int o = ff.boundary_bs[i];
-                const double2 p = ff.boundary_p[i];
-                const double4 pl = ff.planes[ff.boundary_plane[i]];
-                const V3 c = P(o);
-                if constexpr (E) acc[0] += boundary_energy<double>(pl, c, p.x, p.y);
-                if constexpr (F) {
-                    const R f0 = boundary_force_mag<R>(pl, c, p.x, p.y);
-                    target_add(t, f, o, f0 * R(pl.x), f0 * R(pl.y), f0 * R(pl.z));
-                }
-            }
-            break;
-    }
+    chain_lane<R, E, F>(cprev, c, cnext, fl, r.lp, r.bp, own, q, a.t, f, acc[0], acc[1]);
 }
 
 // Bonded chunk b of the main kernel: blockDim records of one segment.
@@ -778,29 +672,7 @@ __global__ void __launch_bounds__(kChainThreads + 32) k_pass_chain(const __grid_
                      cn = stage_pos<LS>(st, j + 2, lam);
             const double2 lp = st.lp[j], bp = st.bp[j];
             const bool own = lane >= 1 && lane <= kWarpOut && q < n;
-            if constexpr (F) {
-                T3<R> Fl{0, 0, 0}, A{0, 0, 0}, B{0, 0, 0};
-                if (fl & kLink) Fl = stretch_force<R>(c, cn, lp.x, lp.y);
-                if (fl & kBend) bend_force<R>(diff<R>(cp, c), diff<R>(c, cn), bp.x, bp.y, A, B);
-                const T3<R> Fp = shfl_up3(Fl), Bp = shfl_up3(B), An = shfl_down3(A);
-                if (own) {
-                    // link (q-1, q) acts on q; link (q, q+1) reacts on q; bends
-                    // centred at q-1 (third bead), q (middle), q+1 (first bead)
-                    const double fx =
-                        double(Fp.x) - double(Fl.x) + double(Bp.x) + (double(A.x) - double(B.x)) - double(An.x);
-                    const double fy =
-                        double(Fp.y) - double(Fl.y) + double(Bp.y) + (double(A.y) - double(B.y)) - double(An.y);
-                    const double fz =
-                        double(Fp.z) - double(Fl.z) + double(Bp.z) + (double(A.z) - double(B.z)) - double(An.z);
-                    target_add(a.t, f, 3 * q, fx, fy, fz);
-                }
-            }
-            if constexpr (E) {
-                if (own) {
-                    if (fl & kLink) acc[0] += stretch_energy<double>(c, cn, lp.x, lp.y);
-                    if (fl & kBend) acc[1] += bend_energy<double>(diff<double>(cp, c), diff<double>(c, cn), bp.x, bp.y);
-                }
-            }
+            chain_lane<R, E, F>(cp, c, cn, fl, lp, bp, own, q, a.t, f, acc[0], acc[1]);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + k);
         }
@@ -819,55 +691,7 @@ __global__ void __launch_bounds__(kPassThreads) k_pass_branch(const __grid_const
     const DeviceFF& ff = a.ff;
     double acc[kBranchVals] = {0.0, 0.0, 0.0, 0.0};
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ff.n_branch) {
-        const int4 q = ff.branch_bs[i];
-        const double4 pa = ff.branch_pa[i], pb = ff.branch_pb[i];
-        const V3 c1 = P(q.x), c2 = P(q.y), c3 = P(q.z), c4 = P(q.w);
-        const int m = ff.branch_mask;
-        if constexpr (E) {
-            if (m & 1) acc[0] += branch_stretch_energy<double>(c1, c2, c3, pa.y, pa.z, pa.x);
-            if (m & 2) acc[1] += bend_energy<double>(diff<double>(c1, c2), diff<double>(c3, c4), pa.w, pb.x);
-            if (m & 4) acc[2] += branch_dihedral_energy<double>(c1, c2, c3, c4, pb.y, pa.x);
-            if (m & 8) acc[3] += branch_position_energy<double>(c1, c2, c3, pb.z, pa.x);
-        }
-        if constexpr (F) {
-            T3<R> F1{0, 0, 0}, F2{0, 0, 0}, F3{0, 0, 0}, F4{0, 0, 0};
-            if (m & 1) {
-                const T3<R> g = branch_stretch_force<R>(c1, c2, c3, pa.y, pa.z, pa.x);
-                const R pm1 = R(pa.x) - R(1), pp = R(pa.x);
-                F1.x += -g.x * pm1; F1.y += -g.y * pm1; F1.z += -g.z * pm1;
-                F2.x += g.x * pp; F2.y += g.y * pp; F2.z += g.z * pp;
-                F3.x += -g.x; F3.y += -g.y; F3.z += -g.z;
-            }
-            if (m & 2) {
-                T3<R> Fr1, Fr2;
-                bend_force<R>(diff<R>(c1, c2), diff<R>(c3, c4), pa.w, pb.x, Fr1, Fr2);
-                F1.x += -Fr1.x; F1.y += -Fr1.y; F1.z += -Fr1.z;
-                F2.x += Fr1.x; F2.y += Fr1.y; F2.z += Fr1.z;
-                F3.x += -Fr2.x; F3.y += -Fr2.y; F3.z += -Fr2.z;
-                F4.x += Fr2.x; F4.y += Fr2.y; F4.z += Fr2.z;
-            }
-            if (m & 4) {
-                T3<R> L1, L2, L3, L4;
-                branch_dihedral_force<R>(c1, c2, c3, c4, pb.y, pa.x, L1, L2, L3, L4);
-                F1.x += L1.x; F1.y += L1.y; F1.z += L1.z;
-                F2.x += L2.x; F2.y += L2.y; F2.z += L2.z;
-                F3.x += L3.x; F3.y += L3.y; F3.z += L3.z;
-                F4.x += L4.x; F4.y += L4.y; F4.z += L4.z;
-            }
-            if (m & 8) {
-                T3<R> P1, P2, P3;
-                branch_position_force<R>(c1, c2, c3, pb.z, pa.x, P1, P2, P3);
-                F1.x += P1.x; F1.y += P1.y; F1.z += P1.z;
-                F2.x += P2.x; F2.y += P2.y; F2.z += P2.z;
-                F3.x += P3.x; F3.y += P3.y; F3.z += P3.z;
-            }
-            target_add(a.t, f, q.x, F1.x, F1.y, F1.z);
-            target_add(a.t, f, q.y, F2.x, F2.y, F2.z);
-            target_add(a.t, f, q.z, F3.x, F3.y, F3.z);
-            target_add(a.t, f, q.w, F4.x, F4.y, F4.z);
-        }
-    }
+    if (i < ff.n_branch) branch_record<R, E, F>(ff, a.t, P, f, i, acc);
     if constexpr (E) block_done<1, E, F>(a, acc, a.row_branch + blockIdx.x, false);
     PASS_TRACE_END(1 + (E ? 10 : 0))
 }
