@@ -522,11 +522,11 @@ medyan_status medyan_mech_hessian(medyan_mech* h, float delta, double* H);
 /* Batched minimization of independent networks                              */
 /* ------------------------------------------------------------------------ */
 /* No counterpart in the reference (which minimizes one system at a time).
-   A batch holds one handle per replica network. medyan_batch_minimize
-   enqueues every replica's whole minimization (one graph launch each, loops
-   on the device) before waiting for any, so the replicas run concurrently and
-   each stops at its own convergence test; every replica gets exactly the
-   CGMethod::minimize semantics of medyan_cg_minimize. */
+   A batch holds one handle per replica network. medyan_batch_minimize runs
+   all replicas concurrently, each to its own convergence test, with exactly
+   the CGMethod::minimize semantics of medyan_cg_minimize: one kernel whose
+   thread-block clusters take a replica each, or, for batches with large
+   replicas, kernels that launch once per pass for the whole packed batch. */
 typedef struct medyan_batch medyan_batch;
 
 medyan_status medyan_batch_create(const medyan_system* systems, int32_t n_replicas, int32_t precision,
@@ -555,8 +555,8 @@ medyan_status medyan_batch_set_deterministic(medyan_batch* b, int32_t on);
 medyan_status medyan_batch_evaluate(medyan_batch* b, const double* const* coords, double* e_totals,
                                     double* const* forces_out);
 
-/* Shapes of a batch's packed layout (each replica's records are padded to
-   whole blocks, so small replicas favour small blocks). Defaults 256, 64,
+/* Shapes of a batch's packed layout, which the autotuner times and batches
+   with large replicas run in (each replica's records are padded to whole blocks, so small replicas favour small blocks). Defaults 256, 64,
    256, 256. Setting them repacks on the next batched call. */
 typedef struct medyan_batch_shapes {
     int32_t bonded_threads;         /* 128, 256, 512 */

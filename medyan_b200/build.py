@@ -24,7 +24,7 @@ LIB = os.path.join(HERE, "libmedyan_b200.so")
 BUILD_TRACE = os.path.join(HERE, "_build_trace")
 LIB_TRACE = os.path.join(HERE, "libmedyan_b200_trace.so")
 
-SOURCES = ["capi.cu", "ff_kernels.cu", "chain.cu", "excl_kernels.cu", "nl.cu", "cg.cu", "batch.cu", "pbatch.cu", "diff.cu", "hessian.cu", "aux.cu", "tune.cu", "noalloc.cu", "pass.cu", "async.cu", "vectorize.cu", "cg_loop.cu"]
+SOURCES = ["capi.cu", "ff_kernels.cu", "chain.cu", "excl_kernels.cu", "nl.cu", "cg.cu", "batch.cu", "pbatch.cu", "diff.cu", "hessian.cu", "aux.cu", "tune.cu", "noalloc.cu", "pass.cu", "async.cu", "vectorize.cu", "cg_loop.cu", "cg_loop_wide.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include"),
           "-I" + CSRC, "--expt-relaxed-constexpr", "--fmad=false"]

@@ -6,7 +6,6 @@
 #include <cstring>
 #include <vector>
 
-#include "cg_loop.h"
 #include "handle.h"
 
 using namespace mb;
@@ -424,7 +423,6 @@ medyan_status medyan_mech::init() {
         e = cudaEventCreateWithFlags(&fork.join[k], cudaEventDisableTiming);
     if (e == cudaSuccess) e = init_excl_kernels();
     if (e == cudaSuccess) e = init_pass_kernels();
-    if (e == cudaSuccess) e = init_cg_loop();
     const size_t n3 = 3 * (size_t)n_beads;
     if (e == cudaSuccess) e = x.reserve(n3);
     if (e == cudaSuccess) e = f.reserve(n3);

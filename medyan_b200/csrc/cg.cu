@@ -27,7 +27,7 @@
 // counted as an energy call as in the reference.
 //
 // Networks of up to kLoopBeads beads run the whole minimization as one
-// resident kernel instead (cg_loop.cu); what follows is the form for larger
+// resident kernel instead (cg_loop_kernel.cuh); what follows is the form for larger
 // ones, and what finishes a minimization that met a pair whose energy or force
 // needs a quadrature. The iteration runs as a CUDA graph whose loops are
 // conditional WHILE nodes (line-search passes inside, iterations outside) and
@@ -730,6 +730,7 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     if (e == cudaSuccess && h->cg_team > 0)
         e = h->cg_rows.reserve(loop_erow_doubles(loop_row_count(h->chain, h->ff)) + loop_vrow_doubles(vec_blocks(n3)));
     if (e == cudaSuccess && h->cg_team > 0) e = h->cg_words.reserve(kLoopWords);
+    if (e == cudaSuccess && h->cg_team > 0) e = init_cg_loop();
     if (e != cudaSuccess) return cuda_status(e);
     const size_t bytes = sizeof(double) * (size_t)n3;
     // pinned staging: coordinates in, coordinates and forces out, state, lambda set
@@ -959,6 +960,26 @@ medyan_status cg_batch_time_evaluate(PackedBatch& pb, int prec, int reps, float*
     return MEDYAN_OK;
 }
 
+CGState batch_start_state(const medyan_cg_params* p, int nb) {
+    CGState c{};
+    c.method = p->method;
+    c.try_to_recover = p->try_to_recover;
+    c.energy_call_limit = p->energy_call_limit;
+    c.force_call_limit = p->force_call_limit > 3 * nb ? p->force_call_limit : 3 * nb;
+    c.max_dist = p->max_dist;
+    c.lambda_max = p->lambda_max;
+    c.grad_tol = p->grad_tol;
+    c.energy_rel_tol = p->energy_rel_tol;
+    c.ls_quad = p->line_search;
+    c.full_passes = 1;
+    c.status = MEDYAN_OK;
+    c.parity = 1;
+    c.grad_inf_norm = __builtin_inf();
+    c.energy_rel_change = __builtin_inf();
+    c.min_e = __builtin_inf();
+    return c;
+}
+
 // Batched CGMethod::minimize over the packed replicas; see the kernels above.
 medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p) {
     const int R = pb.R;
@@ -983,26 +1004,7 @@ medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p)
     if (e != cudaSuccess) return cuda_status(e);
 
     std::vector<CGState> s0(R);
-    for (int r = 0; r < R; ++r) {
-        CGState& c = s0[r];
-        c = CGState{};
-        const int nbr = pb.base[r + 1] - pb.base[r];
-        c.method = p->method;
-        c.try_to_recover = p->try_to_recover;
-        c.energy_call_limit = p->energy_call_limit;
-        c.force_call_limit = p->force_call_limit > 3 * nbr ? p->force_call_limit : 3 * nbr;
-        c.max_dist = p->max_dist;
-        c.lambda_max = p->lambda_max;
-        c.grad_tol = p->grad_tol;
-        c.energy_rel_tol = p->energy_rel_tol;
-        c.ls_quad = p->line_search;
-        c.full_passes = 1;
-        c.status = MEDYAN_OK;
-        c.parity = 1;
-        c.grad_inf_norm = __builtin_inf();
-        c.energy_rel_change = __builtin_inf();
-        c.min_e = __builtin_inf();
-    }
+    for (int r = 0; r < R; ++r) s0[r] = batch_start_state(p, pb.base[r + 1] - pb.base[r]);
     LambdaSet z{};
     z.K = 1;
     const double one = 1.0;

@@ -1,817 +1,20 @@
-// cg_loop.cu — CGMethod::minimize (src/Mechanics/Minimizer/CGMethod.hpp:826-1743)
-// as one resident kernel.
-//
-// A team of blocks (a thread-block cluster, or a cooperative grid) keeps
-// running from the first energy to the last: every step of an iteration is a
-// phase of the kernel, and a team barrier stands where the graph loop (cg.cu)
-// has kernel boundaries. An iteration whose line search takes the predicted
-// trial has two:
-//
-//   pass   energies at the trial step sizes, and the forces at the trial the
-//          previous line search took, side by side                  | barrier
-//   dots   every block adds the energy rows and decides; then, per component,
-//          d = F + beta d, x += lambda d, and the sums F'.F', F'.F, d.F',
-//          max|F'| of the new force F'                              | barrier
-//
-// and the next pass begins with every block adding the rows of the sums. The
-// direction F' + beta d is not stored before the next dots phase: a pass forms
-// it where it gathers a bead (x, F' and d instead of x and d), which saves the
-// direction's own phase. Its slope d.F is F'.F' + beta d.F'; the slope only
-// enters comparisons.
-//
-// No block waits for another's decision: thread 0 of each block runs the same
-// scalar code (cg_scalar.cuh) on the same sums, on the block's own copy of the
-// state in shared memory, so a barrier is all the blocks exchange.
-//
-// The path is the graph loop's bit for bit with deterministic force sums: the
-// potentials are the same expressions, the vector sums that beta is made of
-// keep the order of the vector passes (vec_blocks), and energies are added in
-// the order of the energy kernels and their finish (a deep line search compares
-// energies that differ by their last bits). Only the slope is summed otherwise,
-// and it only enters comparisons with differences of energies.
-//
-// What it leaves to the graph loop: a pair that the analytic excluded-volume
-// formulas reject. Its quadrature is long and rare, so the loop stops in front
-// of the pass and hands its state over.
-#include "cg_loop.h"
-#include "cg_scalar.cuh"
-#include "excl_quad.cuh"
-#include "records.cuh"
+// cg_loop.cu — the resident minimizer loop on blocks of 256 threads, and the
+// rules that choose where a minimization runs.
+#define LOOP_THREADS 256
+#include "cg_loop_kernel.cuh"
+
+#include <mutex>
 
 namespace mb {
-namespace {
-
-constexpr int kWarps = kLoopThreads / 32;
-constexpr int kSlots = MEDYAN_FF_COUNT;
-constexpr int kRowVals = 4;                             // energies of a row: a branch row's four potentials
-constexpr int kFinishShares = kFinishBlocks;            // shares of the rows that the energy finish adds apart
-constexpr int kMaxRows = kFinishShares * 256;           // rows that a share adds in one round
-constexpr int kVecGroups = kLoopThreads / kVecThreads;  // virtual blocks a block works on at once
-constexpr int kVecSlots = 8;                            // and between two barriers of the block
-// Polls before a grid barrier gives up (a poll is one L2 round trip, so this
-// is tens of seconds; blocks are resident together and arrive in microseconds).
-constexpr int kBarrierPolls = 1 << 25;
-
-// Kinds of work in a pass. Rows are in the energy kernels' order: chain,
-// leftover stretches and bends, linkers, motors, branch points, boundary terms,
-// cylinder pairs.
-enum { FX, FB, FC, FLinker, FMotor, FBoundary, FStretch, FBend, kFKinds };
-enum { EX, EC, EB, ELinker, EMotor, EBoundary, EStretch, EBend, kEKinds };
-
-// First energy slot and energies of a row of each kind, four bits apiece (a row
-// beyond the last has none).
-constexpr unsigned long long kSlot0 = (unsigned long long)MEDYAN_FF_EXCLUDED_VOLUME << (4 * EX) |
-                                      (unsigned long long)MEDYAN_FF_FILAMENT_STRETCHING << (4 * EC) |
-                                      (unsigned long long)MEDYAN_FF_BRANCHING_STRETCHING << (4 * EB) |
-                                      (unsigned long long)MEDYAN_FF_LINKER_STRETCHING << (4 * ELinker) |
-                                      (unsigned long long)MEDYAN_FF_MOTOR_STRETCHING << (4 * EMotor) |
-                                      (unsigned long long)MEDYAN_FF_BOUNDARY << (4 * EBoundary) |
-                                      (unsigned long long)MEDYAN_FF_FILAMENT_STRETCHING << (4 * EStretch) |
-                                      (unsigned long long)MEDYAN_FF_FILAMENT_BENDING << (4 * EBend);
-constexpr unsigned long long kVals = 1ull << (4 * EX) | 2ull << (4 * EC) | 4ull << (4 * EB) | 1ull << (4 * ELinker) |
-                                     1ull << (4 * EMotor) | 1ull << (4 * EBoundary) | 1ull << (4 * EStretch) |
-                                     1ull << (4 * EBend);
-
-// Rows (blocks of the energy kernels) of one kind.
-__host__ __device__ inline int loop_rows(const ChainDev& ch, const DeviceFF& ff, int kind) {
-    const int n = kind == EX ? ff.n_excl : kind == EC ? ch.n_pos : kind == EB ? ff.n_branch : kind == ELinker ? ff.n_linker
-                : kind == EMotor ? ff.n_motor : kind == EBoundary ? ff.n_boundary : kind == EStretch ? ff.n_stretch : ff.n_bend;
-    const int per = kind == EX ? kExclBlock : kBlock, b = (n + per - 1) / per;
-    return kind == EC && b > 148 * 4 ? 148 * 4 : b;  // the chain kernel's grid is capped (chain_blocks)
-}
-static_assert(kBlock == kVecThreads && kExclBlock == 64, "the rounds of a pass make the energy kernels' rows");
-
-struct Team {
-    int rank, size;
-    bool cluster;
-    unsigned* bar;
-    unsigned target;  // thread 0: arrivals that end the current grid barrier
-};
-
-// A block's shared memory. The arguments are here too: a team barrier drops
-// what the L1 cache holds, so fields read through a reference to the kernel's
-// parameters would come from the L2 cache after every one.
-struct Smem {
-    LoopArgs a;
-    Team tm;
-    CGState s;
-    LambdaSet L;
-    int rows[kEKinds], row0[kEKinds];   // rows of each energy kind, and the first of them
-    int n_rows;
-    unsigned char row_kind[kMaxRows];
-    double esum[2][kWarps][kRowVals];   // warp sums of an energy round (rounds alternate)
-    double part[kMaxLambda * kSlots][kFinishShares * 8];  // sums over 32 rows each, per step size and slot
-    double out[kMaxLambda * kOut];  // energies per step size: slots, then the total
-    alignas(16) double red[4 * 8];
-    alignas(16) double vred[kVecSlots][8][4];   // warp sums of the virtual blocks in flight
-    double beta;      // the direction is F + beta d
-    int spec_on;      // the next pass computes the speculative force
-    int dirty;        // the next force buffer holds a speculative force
-    int hit;          // the speculative force is the one the iteration needs
-    int min_pending;  // x is the lowest-energy point and not yet copied to min_e
-    int lost;         // a grid barrier gave up
-};
-
-__device__ __forceinline__ Smem& smem() {
-    extern __shared__ __align__(16) unsigned char loop_smem[];
-    return *reinterpret_cast<Smem*>(loop_smem);
-}
-
-// Team barrier: what any thread of the team wrote before it is visible to all
-// after it. False when a grid barrier gave up (the kernel then ends).
-__device__ __forceinline__ bool team_sync() {
-    Smem& sm = smem();
-    Team& t = sm.tm;
-    if (t.cluster) {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        return true;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        t.target += t.size;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
-        unsigned v = 0;
-        int polls = 0;
-        do {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(t.bar) : "memory");
-        } while ((int)(v - t.target) < 0 && ++polls < kBarrierPolls);
-        if ((int)(v - t.target) < 0) sm.lost = 1;
-    }
-    __syncthreads();
-    return !sm.lost;
-}
-
-// Positions x, or x + lam (F + beta d), of arrays that change during the
-// kernel: plain loads.
-struct Pos {
-    const double* x;
-    const double* d;
-    const double* F;
-    double beta, lam;
-    bool move;
-    __device__ __forceinline__ V3 operator()(int o) const {
-        const V3 p{x[o], x[o + 1], x[o + 2]};
-        if (!move) return p;
-        const V3 g{F[o], F[o + 1], F[o + 2]}, q{d[o], d[o + 1], d[o + 2]};
-        return move3(p, lam, V3{g.x + beta * q.x, g.y + beta * q.y, g.z + beta * q.z});
-    }
-};
-
-// Force target with the kind of sums fixed at compile time: half the code of
-// every addition, in a kernel that is bound by fetching its instructions.
-template <bool FIXED>
-struct Sink {
-    int* status;
-};
-template <bool FIXED, class R>
-__device__ __forceinline__ void target_add(const Sink<FIXED>& t, double* f, int off, R fx, R fy, R fz) {
-    if constexpr (FIXED) {
-        red_add_fixed(f + off, fixed_of(double(fx), t.status));
-        red_add_fixed(f + off + 1, fixed_of(double(fy), t.status));
-        red_add_fixed(f + off + 2, fixed_of(double(fz), t.status));
-    } else {
-        add_force(f, off, fx, fy, fz);
-    }
-}
-
-// Chain tile w: lanes hold centres 30w-1 .. 30w+30.
-template <class R, bool E, bool F, class Target>
-__device__ __forceinline__ void chain_tile(const ChainDev& ch, const Target& t, const Pos& P, double* f, int w,
-                                           double& es, double& eb) {
-    const int n = ch.n_pos, lane = threadIdx.x & 31;
-    const int q = w * kWarpOut - 1 + lane;
-    const bool in = q >= 0 && q < n;
-    const int qe = lane == 0 ? q - 1 : q + 1;
-    V3 c{0.0, 0.0, 0.0}, ce{0.0, 0.0, 0.0};
-    if (in) c = P(3 * q);
-    if ((lane == 0 || lane == 31) && qe >= 0 && qe < n) ce = P(3 * qe);
-    const unsigned fl = in ? __ldg(ch.flags + q) : 0u;
-    const double2 lp = in ? __ldg(ch.link_p + q) : double2{0.0, 0.0};
-    const double2 bp = in ? __ldg(ch.bend_p + q) : double2{0.0, 0.0};
-    V3 cprev = shfl_up3(c), cnext = shfl_down3(c);
-    if (lane == 0) cprev = ce;
-    if (lane == 31) cnext = ce;
-    chain_lane<R, E, F>(cprev, c, cnext, fl, lp, bp, lane >= 1 && lane <= kWarpOut && in, q, t, f, es, eb);
-}
-
-// Energies of the link and the bend of position q (32 consecutive positions
-// per warp).
-__device__ __forceinline__ void chain_energies(const ChainDev& ch, const Pos& P, int q, double& es, double& eb) {
-    const int n = ch.n_pos, lane = threadIdx.x & 31;
-    const bool in = q < n;
-    const int qe = lane == 0 ? q - 1 : q + 1;
-    V3 c{0.0, 0.0, 0.0}, ce{0.0, 0.0, 0.0};
-    if (in) c = P(3 * q);
-    if ((lane == 0 || lane == 31) && qe >= 0 && qe < n) ce = P(3 * qe);
-    const unsigned fl = in ? __ldg(ch.flags + q) : 0u;
-    const double2 lp = in ? __ldg(ch.link_p + q) : double2{0.0, 0.0};
-    const double2 bp = in ? __ldg(ch.bend_p + q) : double2{0.0, 0.0};
-    V3 cp = shfl_up3(c), cn = shfl_down3(c);
-    if (lane == 0) cp = ce;
-    if (lane == 31) cn = ce;
-    if (fl & kLink) es += stretch_energy<double>(c, cn, lp.x, lp.y);
-    if (fl & kBend) eb += bend_energy<double>(diff<double>(cp, c), diff<double>(c, cn), bp.x, bp.y);
-}
-
-__device__ __forceinline__ double tree8(const double (*v)[kRowVals], int j) {
-    return ((v[0][j] + v[4][j]) + (v[2][j] + v[6][j])) + ((v[1][j] + v[5][j]) + (v[3][j] + v[7][j]));
-}
-
-// One pass: energies at the K step sizes of sm.L into the energy rows, and,
-// with force, the forces at lam_f added to f. P gives the positions (at x
-// itself without a move).
-//
-// Forces are cut into warp tasks: eight cylinder pairs, 32 records, or a chain
-// tile. Energies are cut into rounds, in which the block's eight warps make one
-// row: the 256 records, 256 positions or 64 pairs whose energies a block of the
-// energy kernels adds, in its order. Tasks and rounds are numbered by kind,
-// the long kinds first; consecutive tasks go to the warps of one block, and the
-// rounds follow on the blocks after the tasks. An SM so executes few kinds in a
-// pass: the kernel's code is several times an SM's instruction cache, and with
-// kinds dealt round the blocks a task spent half its time fetching
-// instructions (a pass of 2000 filaments of 20 cylinders 13.2 against 11.9 us).
-template <class R, bool FIXED>
-__device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double* f, int* status, int parity) {
-    Smem& sm = smem();
-    const LoopArgs& a = sm.a;
-    const Team& tm = sm.tm;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3;
-    const DeviceFF& ff = a.ff;
-    const Sink<FIXED> t{status};
-    bool bad = false;
-    int f_blocks = 0;  // blocks that the force tasks fill
-    if (force) {
-        // lane l: tasks of kind l, and the end of their numbers
-        const int n = lane == FX ? ff.n_excl : lane == FB ? ff.n_branch : lane == FC ? a.ch.n_pos : lane == FLinker ? ff.n_linker
-                    : lane == FMotor ? ff.n_motor : lane == FBoundary ? ff.n_boundary : lane == FStretch ? ff.n_stretch
-                    : lane == FBend ? ff.n_bend : 0;
-        const int per = lane == FX ? 8 : lane == FC ? kWarpOut : 32;
-        int end = (n + per - 1) / per;
-#pragma unroll
-        for (int o = 1; o < kFKinds; o <<= 1) {
-            const int v = __shfl_up_sync(kFull, end, o);
-            if (lane >= o) end += v;
-        }
-        const int total = __shfl_sync(kFull, end, kFKinds - 1);
-        f_blocks = (total + kWarps - 1) / kWarps;
-        P.lam = lam_f;
-#pragma unroll 1
-        for (int task = tm.rank * kWarps + warp; task < total; task += tm.size * kWarps) {
-            const int kind = __popc(__ballot_sync(kFull, end <= task) & ((1u << kFKinds) - 1u));
-            const int before = __shfl_sync(kFull, end, kind > 0 ? kind - 1 : 0);
-            const int i = kind > 0 ? task - before : task;
-            double none[4];
-            if (kind == FX) {
-                const int p = i * 8 + (lane >> 2), pc = min(p, ff.n_excl - 1);
-                const int4 q = __ldg(ff.excl_bs + pc);
-                const double krs = __ldg(ff.excl_krs + pc);
-                // lane j of a pair fetches bead j and gets the force on it
-                const int o = quad < 2 ? (quad == 0 ? q.x : q.y) : (quad == 2 ? q.z : q.w);
-                const V3 own = P(o);
-                T3<double> fo;
-                const bool ok = excl_force_quad<sizeof(R) == 8>(quad, quad_lane3(own, 0), quad_lane3(own, 1),
-                                                                quad_lane3(own, 2), quad_lane3(own, 3), krs, fo);
-                if (p < ff.n_excl) {
-                    if (ok) target_add(t, f, o, fo.x, fo.y, fo.z);
-                    else bad = true;
-                }
-            } else if (kind == FB) {
-                if (i * 32 + lane < ff.n_branch) branch_record<R, false, true>(ff, t, P, f, i * 32 + lane, none);
-            } else if (kind == FC) {
-                chain_tile<R, false, true>(a.ch, t, P, f, i, none[0], none[1]);
-            } else {
-                const int seg = kind < FBoundary ? kind - FLinker + 2 : kind == FBoundary ? 5 : kind - FStretch;
-                bonded_record<R, false, true>(ff, t, P, f, seg, i * 32 + lane, none);
-            }
-        }
-    }
-    if (K > 0) {
-        int rounds = sm.n_rows * K, alt = 0;
-        int first = (tm.rank - f_blocks) % tm.size;
-        if (first < 0) first += tm.size;
-#pragma unroll 1
-        for (int round = first; round < rounds; round += tm.size, alt ^= 1) {
-            int kind = 0, v = round, k = 0;
-            while (v >= sm.rows[kind] * K) v -= sm.rows[kind++] * K;
-            while (v >= sm.rows[kind]) {
-                v -= sm.rows[kind];
-                ++k;
-            }
-            P.lam = sm.L.lam[k];
-            double e[kRowVals] = {0.0, 0.0, 0.0, 0.0};
-            const int i = v * kVecThreads + threadIdx.x;  // record or position of this thread
-            if (kind == EX) {
-                // 64 pairs: warp 4c + j takes the pairs j, j + 4, ... of 32-pair
-                // chunk c, which are those the chunk's sum joins first
-                const int p = v * 64 + (warp >> 2) * 32 + (warp & 3) + (lane & ~3), pc = min(p, ff.n_excl - 1);
-                const int4 q = __ldg(ff.excl_bs + pc);
-                const double krs = __ldg(ff.excl_krs + pc);
-                const V3 own = P(quad < 2 ? (quad == 0 ? q.x : q.y) : (quad == 2 ? q.z : q.w));
-                const double U = excl_energy_quad(quad, quad_lane3(own, 0), quad_lane3(own, 1), quad_lane3(own, 2),
-                                                  quad_lane3(own, 3), krs);
-                if (p < ff.n_excl) {
-                    if (excl_energy_bad(U)) bad = true;
-                    e[0] = U;
-                }
-            } else if (kind == EC) {
-                for (int q = i; q - lane < a.ch.n_pos; q += sm.rows[EC] * kVecThreads)
-                    chain_energies(a.ch, P, q, e[0], e[1]);
-            } else if (kind == EB) {
-                if (i < ff.n_branch) branch_record<double, true, false>(ff, t, P, f, i, e);
-            } else {
-                const int seg = kind < EBoundary ? kind - ELinker + 2 : kind == EBoundary ? 5 : kind - EStretch;
-                bonded_record<double, true, false>(ff, t, P, f, seg, i, e);
-            }
-            const int vals = kind == EB ? 4 : kind == EC ? 2 : 1;
-#pragma unroll
-            for (int j = 0; j < kRowVals; ++j) {
-                if (j < vals) {
-#pragma unroll
-                    for (int o = 16; o > 2; o >>= 1) e[j] += __shfl_down_sync(kFull, e[j], o);
-                    if (kind != EX) {
-                        e[j] += __shfl_down_sync(kFull, e[j], 2);
-                        e[j] += __shfl_down_sync(kFull, e[j], 1);
-                    }
-                    if (lane == 0) sm.esum[alt][warp][j] = e[j];
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x < vals) {
-                const double(*w)[kRowVals] = sm.esum[alt];
-                const double sum = kind != EX ? tree8(w, threadIdx.x)
-                                              : ((w[0][0] + w[2][0]) + (w[1][0] + w[3][0])) +
-                                                    ((w[4][0] + w[6][0]) + (w[5][0] + w[7][0]));
-                a.erow[((size_t)(parity * kMaxLambda + k) * kRowVals + threadIdx.x) * sm.n_rows + sm.row0[kind] + v] = sum;
-            }
-        }
-    }
-    if (bad) atomicOr(a.words + parity, 1);
-}
-
-// After the barrier that follows a pass: whether it met a pair that needs a
-// quadrature (the same answer in every block: the flag of this parity is not
-// written again before the next barrier), and else the energies: every block
-// adds the rows in the order of the energy finish (k_energy_finish: eight
-// shares of the rows; in a share, a tree over 32 rows, a tree over eight such
-// sums; then the shares in order) and applies
-// ForceFieldManager::computeEnergy's rule (a force field at or below -1 makes
-// the total +inf, ForceFieldManager.cpp:137-176).
-__device__ __noinline__ bool add_rows(int K, int parity) {
-    Smem& sm = smem();
-    const LoopArgs& a = sm.a;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int flag = *reinterpret_cast<volatile int*>(a.words + parity);
-    const int R = sm.n_rows, share = (R + kFinishShares - 1) / kFinishShares, subs = (share + 31) / 32;
-#pragma unroll 1
-    for (int item = warp; item < K * kFinishShares * subs; item += kWarps) {
-        const int u = item % subs, b = item / subs % kFinishShares, k = item / subs / kFinishShares;
-        const int r = b * share + u * 32 + lane;
-        const int kind = r < R && r < (b + 1) * share ? sm.row_kind[r] : kEKinds;
-        const int slot0 = (int)(kSlot0 >> (4 * kind)) & 15, vals = (int)(kVals >> (4 * kind)) & 15;
-        const double* row = a.erow + (size_t)(parity * kMaxLambda + k) * kRowVals * R + r;
-        double v[kRowVals], mine = 0.0;
-#pragma unroll
-        for (int j = 0; j < kRowVals; ++j) v[j] = j < vals ? row[(size_t)j * R] : 0.0;
-        // a tree over the 32 rows for each slot that one of them has; lane s keeps slot s
-        unsigned slots = __reduce_or_sync(kFull, ((1u << vals) - 1u) << slot0);
-#pragma unroll 1
-        for (; slots; slots &= slots - 1u) {
-            const int slot = __ffs(slots) - 1, j = slot - slot0;
-            double w = j < 0 || j >= vals ? 0.0 : (j < 2 ? (j == 0 ? v[0] : v[1]) : (j == 2 ? v[2] : v[3]));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(kFull, w, o);
-            w = __shfl_sync(kFull, w, 0);
-            if (lane == slot) mine = w;
-        }
-        if (lane < kSlots) sm.part[k * kSlots + lane][b * 8 + u] = mine;
-    }
-    if (__syncthreads_or(flag)) return false;
-    // eight lanes per step size and slot: a share each, then the shares in order
-#pragma unroll 1
-    for (int i0 = warp * 32; i0 < K * kSlots * kFinishShares; i0 += kLoopThreads) {
-        const int c = min((i0 + lane) >> 3, K * kSlots - 1), b = lane & 7;
-        const double* q = sm.part[c] + 8 * b;
-        double w = q[0];
-        if (subs > 1) {
-            double z[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) z[u] = u < subs ? q[u] : 0.0;
-            w = ((z[0] + z[4]) + (z[2] + z[6])) + ((z[1] + z[5]) + (z[3] + z[7]));
-        }
-        double v = 0.0;
-#pragma unroll
-        for (int q8 = 0; q8 < kFinishShares; ++q8) v += __shfl_sync(kFull, w, q8, 8);
-        if (b == 0) sm.out[c / kSlots * kOut + c % kSlots] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-        double* o = sm.out + threadIdx.x * kOut;
-        double tot = 0.0;
-        bool inf = false;
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s) {
-            if (o[s] <= -1) inf = true;
-            else tot += o[s];
-        }
-        o[kSlots] = inf ? __longlong_as_double(0x7ff0000000000000ULL) : tot;
-    }
-    __syncthreads();
-    return true;
-}
-
-// Sums and a maximum of a vector pass: F'.F', F'.F, d.F', max|F'|.
-struct Sums {
-    double a, b, c, m;
-};
-__device__ __forceinline__ void join(Sums& s, const Sums& o) {
-    s.a += o.a;
-    s.b += o.b;
-    s.c += o.c;
-    s.m = dmax_ref(s.m, o.m);
-}
-// Lane 0 gets the warp's, by the tree of the vector passes.
-__device__ __forceinline__ void warp_join(Sums& s) {
-#pragma unroll 1
-    for (int o = 16; o > 0; o >>= 1) {
-        Sums n;
-        n.a = __shfl_down_sync(kFull, s.a, o);
-        n.b = __shfl_down_sync(kFull, s.b, o);
-        n.c = __shfl_down_sync(kFull, s.c, o);
-        n.m = __shfl_down_sync(kFull, s.m, o);
-        join(s, n);
-    }
-}
-// The same tree over eight warps' sums, by the lanes of a group of eight (all
-// 32 lanes call; valid in the group's first lane).
-__device__ __forceinline__ void eight_join(Sums& s) {
-#pragma unroll 1
-    for (int o = 4; o > 0; o >>= 1) {
-        Sums n;
-        n.a = __shfl_down_sync(kFull, s.a, o, 8);
-        n.b = __shfl_down_sync(kFull, s.b, o, 8);
-        n.c = __shfl_down_sync(kFull, s.c, o, 8);
-        n.m = __shfl_down_sync(kFull, s.m, o, 8);
-        join(s, n);
-    }
-}
-__device__ __forceinline__ void put(double* r, const Sums& s) {
-    *reinterpret_cast<double2*>(r) = double2{s.a, s.b};
-    *reinterpret_cast<double2*>(r + 2) = double2{s.c, s.m};
-}
-__device__ __forceinline__ Sums get(const double* r) {
-    const double2 p = *reinterpret_cast<const double2*>(r), q = *reinterpret_cast<const double2*>(r + 2);
-    return Sums{p.x, p.y, q.x, q.y};
-}
-
-// One vector pass: load(i) for every component i, then apply(i, loaded, sums).
-// A virtual block of 256 threads (vec_blocks) is worked by eight warps of one
-// block; with a single virtual block its warps are spread over the team
-// instead. Its sums go to a row.
-template <class Load, class Apply>
-__device__ __forceinline__ void vector_pass(double* rows, Load load, Apply apply) {
-    Smem& sm = smem();
-    const LoopArgs& a = sm.a;
-    const Team& tm = sm.tm;
-    constexpr int kAhead = 2;  // components loaded before the first is used
-    const int lane = threadIdx.x & 31, stride = a.vb * kVecThreads;
-    const bool one = a.vb == 1;
-    const int t = threadIdx.x % kVecThreads, g = threadIdx.x / kVecThreads;
-    // units: virtual blocks (a group of eight warps each), or warps of the only one
-    const int units = one ? 8 : a.vb, per = one ? tm.size * kWarps : tm.size * kVecGroups;
-    const int mine = one ? tm.rank * kWarps + (threadIdx.x >> 5) : tm.rank * kVecGroups + g;
-    const int most = kVecSlots / kVecGroups;
-    for (int u0 = mine - (one ? 0 : g); u0 < units; u0 += per * most) {
-#pragma unroll 1
-        for (int k = 0; k < most && u0 + k * per + (one ? 0 : g) < units; ++k) {
-            const int u = u0 + k * per + (one ? 0 : g);
-            Sums s{0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-            for (int i = one ? u * 32 + lane : u * kVecThreads + t; i < a.n3; i += kAhead * stride) {
-                decltype(load(0)) v[kAhead];
-#pragma unroll
-                for (int q = 0; q < kAhead; ++q)
-                    if (i + q * stride < a.n3) v[q] = load(i + q * stride);
-#pragma unroll
-                for (int q = 0; q < kAhead; ++q)
-                    if (i + q * stride < a.n3) apply(i + q * stride, v[q], s);
-            }
-            warp_join(s);
-            if (lane == 0) put(one ? rows + 4 * u : sm.vred[k * kVecGroups + g][t >> 5], s);
-        }
-        if (one) continue;
-        __syncthreads();
-        if (threadIdx.x < 8 * kVecSlots) {  // eight lanes per virtual block
-            const int slot = threadIdx.x >> 3, v = u0 + slot / kVecGroups * per + slot % kVecGroups;
-            Sums s = get(sm.vred[slot][threadIdx.x & 7]);
-            eight_join(s);
-            if ((threadIdx.x & 7) == 0 && v < a.vb) put(rows + 4 * (size_t)v, s);
-        }
-        if (u0 + per * most < units) __syncthreads();
-    }
-}
-
-// After the barrier that follows a vector pass: the sums of its rows, in the
-// vector passes' order (thread q adds blocks q, q + 256, ..., then a tree).
-// Valid in thread 0.
-__device__ __noinline__ Sums add_vector_rows(const double* rows) {
-    Smem& sm = smem();
-    const LoopArgs& a = sm.a;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, vb = a.vb;
-    Sums s{0.0, 0.0, 0.0, 0.0};
-    if (vb == 1) {
-        if (warp == 0) {
-            if (lane < 8) s = get(rows + 4 * lane);
-            eight_join(s);
-        }
-        return s;
-    }
-    if (warp * 32 < vb && warp < 8) {
-#pragma unroll 1
-        for (int q = threadIdx.x; q < vb; q += kVecThreads) join(s, get(rows + 4 * (size_t)q));
-        warp_join(s);
-    }
-    if (vb > 32) {
-        if (lane == 0 && warp < 8) put(sm.red + 4 * warp, s);
-        __syncthreads();
-        if (warp == 0) {
-            s = get(sm.red + 4 * (lane & 7));
-            eight_join(s);
-        }
-    }
-    return s;
-}
-
-template <class R, bool FIXED>
-__device__ void minimize() {
-    Smem& sm = smem();
-    const LoopArgs& a = sm.a;
-    const Team& tm = sm.tm;
-    CGState& s = sm.s;
-    auto words = [](auto& v) { return reinterpret_cast<int*>(&v); };
-    for (int i = threadIdx.x; i < (int)(sizeof(CGState) / 4); i += kLoopThreads) words(s)[i] = words(*a.st)[i];
-    if (threadIdx.x == 0) {
-        sm.L = LambdaSet{};
-        sm.L.K = 1;
-        sm.beta = 0.0;
-        sm.spec_on = sm.dirty = sm.hit = sm.min_pending = sm.lost = 0;
-        int at = 0;
-        for (int kind : {EC, EStretch, EBend, ELinker, EMotor, EB, EBoundary, EX}) {
-            sm.rows[kind] = loop_rows(a.ch, a.ff, kind);
-            sm.row0[kind] = at;
-            at += sm.rows[kind];
-        }
-        sm.n_rows = at;
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < sm.n_rows; r += kLoopThreads)
-        for (int kind = 0; kind < kEKinds; ++kind)
-            if (r >= sm.row0[kind] && r < sm.row0[kind] + sm.rows[kind]) sm.row_kind[r] = (unsigned char)kind;
-    __syncthreads();
-    const int first = tm.rank * kLoopThreads + threadIdx.x, step = tm.size * kLoopThreads;
-    int parity = 0;  // of the passes: which energy rows and pass flag the next one uses
-    auto current = [&] { return s.parity ? a.f1 : a.f0; };
-    auto other = [&] { return s.parity ? a.f0 : a.f1; };
-    // Writes the state back (block 0) and ends the kernel with `code`. The
-    // graph loop finds the direction and the lowest-energy point in place.
-    auto leave = [&](int code) {
-        if (code == kLoopHandOver) {
-            const double* F = current();
-            for (int i = first; i < a.n3; i += step) {
-                a.d[i] = F[i] + sm.beta * a.d[i];
-                if (sm.min_pending) a.min_e[i] = a.x[i];
-            }
-        }
-        __syncthreads();
-        if (tm.rank != 0) return;
-        if (threadIdx.x == 0) {
-            s.spec_valid = 0;
-            s.spec_skip = 1;
-            s.force_skip = 0;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < (int)(sizeof(CGState) / 4); i += kLoopThreads) words(*a.st)[i] = words(s)[i];
-        if (threadIdx.x == 0) {
-            *a.lam = sm.L;
-            a.words[2] = code;
-        }
-    };
-    auto record = [&](int which) {
-        if (threadIdx.x == 0) {
-            double tot = 0.0;
-            for (int i = 0; i < kSlots; ++i) tot += sm.out[i];  // computeIndividualEnergies: no -1 rule
-            if (tm.rank == 0) {
-                for (int i = 0; i < kSlots; ++i) a.eout[which * kOut + i] = sm.out[i];
-                a.eout[which * kOut + kSlots] = tot;
-            }
-            s.num_energy_call++;
-            if (which == 0) {
-                s.prev_energy = tot;
-                s.need_e0 = 1;
-            }
-        }
-    };
-    const Pos at_x{a.x, nullptr, nullptr, 0.0, 0.0, false};
-
-    // energies before, and the first force
-    pass<R, FIXED>(at_x, 1, true, 0.0, other(), a.status, parity);
-    if (!team_sync()) return leave(kLoopLost);
-    if (!add_rows(1, parity)) return leave(kLoopRestart);
-    parity ^= 1;
-    record(0);
-    __syncthreads();
-
-    for (;;) {
-        // dots: the direction, the move, the new force's sums; the buffer of
-        // the old force becomes zero for the next one
-        const bool moved = !s.done && !s.skip_force;
-        if (moved) {
-            double *Fn = other(), *Fc = current();
-            const double lam = s.lam_move, beta = sm.beta;
-            const bool copy = sm.min_pending;
-            double *x = a.x, *d = a.d, *min_e = a.min_e;
-            struct In {
-                double x, d, fn, fc;
-            };
-            vector_pass(
-                a.vrow, [&](int i) { return In{x[i], d[i], Fn[i], Fc[i]}; },
-                [&](int i, In v, Sums& q) {
-                    const double dn = v.fc + beta * v.d;  // shiftSearchDir (CGMethod.cpp:356-360)
-                    if (copy) min_e[i] = v.x;
-                    d[i] = dn;
-                    x[i] = move1(v.x, lam, dn);
-                    if constexpr (FIXED) {
-                        v.fn = double(__double_as_longlong(v.fn)) / kFixedScale;
-                        Fn[i] = v.fn;
-                    }
-                    Fc[i] = 0.0;
-                    q.a += v.fn * v.fn;
-                    q.b += v.fn * v.fc;
-                    q.c += dn * v.fn;
-                    q.m = dmax_ref(q.m, fabs(v.fn));
-                });
-            if (tm.rank == 0 && threadIdx.x == 0) a.st->spec_status = 0;
-            if (!team_sync()) return leave(kLoopLost);
-            const Sums q = add_vector_rows(a.vrow);
-            if (threadIdx.x == 0) {
-                sm.min_pending = 0;
-                dots_tail(s, q.a, q.b, q.m);
-                if (s.copy_min_e) sm.min_pending = 1;
-                // d.F of the new direction
-                s.slope = s.dir_mode ? s.new_grad : s.new_grad + s.beta * q.c;
-            }
-        } else {
-            __syncthreads();
-            if (threadIdx.x == 0 && !s.done) s.slope = s.new_grad;  // the line search failed: d = F
-        }
-        __syncthreads();
-        if (s.done) break;
-        if (s.safe_mode) {
-            // max|d|, which only the recovery step after a second failure needs;
-            // its rows are apart: another block may still be adding the sums'. A
-            // failed line search leaves its speculative force in the other
-            // buffer, which the next pass needs zero
-            double* max_rows = a.vrow + loop_vrow_doubles(a.vb) / 2;
-            const double* F = current();
-            const double beta = s.dir_mode ? 0.0 : s.beta;
-            if (!moved)
-                for (int i = first; i < a.n3; i += step) other()[i] = 0.0;
-            struct In {
-                double f, d;
-            };
-            vector_pass(
-                max_rows, [&](int i) { return In{F[i], a.d[i]}; },
-                [&](int, const In& v, Sums& q) { q.m = dmax_ref(q.m, fabs(v.f + beta * v.d)); });
-            if (tm.rank == 0 && threadIdx.x == 0) a.st->spec_status = 0;
-            if (!team_sync()) return leave(kLoopLost);
-            const Sums q = add_vector_rows(max_rows);
-            if (threadIdx.x == 0) s.dmax = q.m;
-        }
-        __syncthreads();  // every thread has read the state that thread 0 now changes
-        if (threadIdx.x == 0) {
-            sm.beta = s.dir_mode ? 0.0 : s.beta;
-            dir_tail(s, sm.L, s.slope, s.dmax);
-            if (s.reset_after_dir) sm.beta = 0.0;  // conjugacy lost: d = F
-            sm.dirty = sm.hit = sm.spec_on = 0;
-            s.spec_valid = 0;
-            // the speculative force: at the trial that the previous line
-            // search took, when the first pass offers it
-            const int j = (s.need_e0 ? 1 : 0) + s.last_backtracks;
-            if (!s.done && !s.ls_immediate_fail && j < sm.L.K) {
-                s.spec_lam = sm.L.lam[j];
-                s.spec_valid = sm.spec_on = sm.dirty = 1;
-            }
-        }
-        __syncthreads();
-        if (s.done) break;
-        // line search
-        const Pos along{a.x, a.d, current(), sm.beta, 0.0, true};
-        while (s.ls_active && !s.done) {
-            const int K = s.ls_immediate_fail ? 0 : sm.L.K;
-            if (K > 0) {
-                pass<R, FIXED>(along, K, sm.spec_on, s.spec_lam, other(), &a.st->spec_status, parity);
-                if (!team_sync()) return leave(kLoopLost);
-                if (!add_rows(K, parity)) return leave(kLoopHandOver);
-                parity ^= 1;
-            } else {
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) {
-                ls_decide(s, sm.L, sm.out);
-                sm.spec_on = 0;
-                if (!s.ls_active) {
-                    sm.hit = s.spec_valid && !s.skip_force && s.lam_move == s.spec_lam;
-                    if (sm.hit && tm.rank == 0 && a.st->spec_status) *a.status |= a.st->spec_status;
-                    s.spec_valid = 0;
-                }
-            }
-            __syncthreads();
-        }
-        // the force at the accepted step, unless the line search's pass had it
-        if (!s.done && !s.skip_force && !sm.hit) {
-            double* F = other();
-            if (sm.dirty) {
-                for (int i = first; i < a.n3; i += step) F[i] = 0.0;
-                if (!team_sync()) return leave(kLoopLost);
-            }
-            pass<R, FIXED>(along, 0, true, s.lam_move, F, a.status, parity);
-            if (!team_sync()) return leave(kLoopLost);
-            if (!add_rows(0, parity)) return leave(kLoopHandOver);
-            parity ^= 1;
-        }
-    }
-
-    // epilogue: the lowest-energy coordinates after a call limit, the current
-    // force into f0, the energies after
-    const bool restore =
-        s.status != MEDYAN_ERR_LINE_SEARCH && s.call_limit && s.have_min_e && !sm.min_pending;
-    const bool copy_f = s.parity != 0;
-    for (int i = first; i < a.n3; i += step) {
-        if (restore) a.x[i] = a.min_e[i];
-        if (copy_f) a.f0[i] = a.f1[i];
-    }
-    if (threadIdx.x == 0) {
-        sm.L.K = 1;
-        sm.L.lam[0] = 0.0;
-    }
-    if (!team_sync()) return leave(kLoopLost);
-    if (s.status != MEDYAN_ERR_LINE_SEARCH) {
-        pass<R, FIXED>(at_x, 1, false, 0.0, nullptr, nullptr, parity);
-        if (!team_sync()) return leave(kLoopLost);
-        if (!add_rows(1, parity)) return leave(kLoopHandOver);
-        record(1);
-        __syncthreads();
-    }
-    leave(kLoopDone);
-}
-
-template <class R, bool FIXED, bool CLUSTER>
-__global__ void __launch_bounds__(kLoopThreads, 1) k_cg_loop(const __grid_constant__ LoopArgs a) {
-    if (threadIdx.x == 0) {
-        smem().a = a;
-        smem().tm = Team{(int)blockIdx.x, (int)gridDim.x, CLUSTER, reinterpret_cast<unsigned*>(a.words + 3), 0u};
-    }
-    __syncthreads();
-    minimize<R, FIXED>();
-}
-
-template <class R, bool FIXED>
-cudaError_t launch(const LoopArgs& a, int team, cudaStream_t s) {
-    cudaLaunchConfig_t c{};
-    c.gridDim = dim3(team);
-    c.blockDim = dim3(kLoopThreads);
-    c.dynamicSmemBytes = sizeof(Smem);
-    c.stream = s;
-    cudaLaunchAttribute at{};
-    c.attrs = &at;
-    c.numAttrs = 1;
-    if (team <= kLoopCluster) {
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = team;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        return cudaLaunchKernelEx(&c, k_cg_loop<R, FIXED, true>, a);
-    }
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    return cudaLaunchKernelEx(&c, k_cg_loop<R, FIXED, false>, a);
-}
-
-template <class R, bool FIXED>
-cudaError_t allow_clusters() {
-    return cudaFuncSetAttribute(k_cg_loop<R, FIXED, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-}
-
-}  // namespace
 
 // Which networks run here, and on how many blocks: one for every eight force
 // tasks and every energy round of a pass with one step size, so that a small
 // network's work all runs at once, up to one block per SM.
 //
 // A cluster's barrier takes 0.7 us where the grid's takes 1.2, so teams of up
-// to 16 blocks (the largest cluster) are clusters. The graph loop takes over at
-// 250,000 beads: its kernels hold three to four times as many threads per SM.
-// Microseconds per iteration here / graph loop (FP64, filaments of 20
-// cylinders): 200 filaments 17 / 66, 2000: 25 / 59, 8000: 55 / 72, 12000: 75 /
-// 81, 20000: 112 / 105.
+// to 16 blocks (the largest cluster) are clusters. The graph loop takes over
+// where its kernels, which hold three to four times as many threads per SM,
+// are faster.
 int loop_team(const ChainDev& ch, const DeviceFF& ff) {
     if (ch.n_pos <= 0 || ch.n_pos > kLoopBeads) return 0;
     auto chunks = [](int n, int per) { return (n + per - 1) / per; };
@@ -832,20 +35,25 @@ int loop_row_count(const ChainDev& ch, const DeviceFF& ff) {
     return n;
 }
 
+size_t loop_erow_doubles(int rows) { return 2 * (size_t)kMaxLambda * kRowVals * rows; }
+
 cudaError_t init_cg_loop() {
-    cudaError_t e = allow_clusters<float, false>();
-    if (e == cudaSuccess) e = allow_clusters<float, true>();
-    if (e == cudaSuccess) e = allow_clusters<double, false>();
-    if (e == cudaSuccess) e = allow_clusters<double, true>();
+    static std::mutex mu;
+    static bool done[64];
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(mu);
+    if (done[dev]) return cudaSuccess;
+    e = allow_clusters<false>();
+    if (e == cudaSuccess) e = init_cg_loop_wide();
+    if (e == cudaSuccess) done[dev] = true;
     return e;
 }
 
-size_t loop_erow_doubles(int rows) { return 2 * (size_t)kMaxLambda * kRowVals * rows; }
-
-
 cudaError_t launch_cg_loop(const LoopArgs& a, int prec, int team, cudaStream_t s) {
-    if (prec == MEDYAN_PREC_MIXED) return a.fixed ? launch<float, true>(a, team, s) : launch<float, false>(a, team, s);
-    return a.fixed ? launch<double, true>(a, team, s) : launch<double, false>(a, team, s);
+    return a.n3 > 3 * kLoopWideBeads ? launch_cg_loop_wide(a, prec, team, s) : launch_single(a, prec, team, s);
 }
 
 }  // namespace mb

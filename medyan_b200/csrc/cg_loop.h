@@ -1,4 +1,4 @@
-// cg_loop.h — the resident minimizer loop (cg_loop.cu): one kernel that runs a
+// cg_loop.h — the resident minimizer loop (cg_loop_kernel.cuh): one kernel that runs a
 // whole CGMethod::minimize on a team of thread blocks.
 #pragma once
 
@@ -28,7 +28,6 @@ struct LoopArgs {
 // words: two pass flags (a pair needs a quadrature fallback), the loop's
 // outcome, the grid barrier's counter.
 constexpr int kLoopWords = 4;
-constexpr int kLoopThreads = 256;
 // words[2] at the end: the minimization is complete; it stopped in the loop
 // and the graph loop takes over from *st; it stopped in the setup, nothing is
 // changed but the force buffers; a grid barrier gave up.
@@ -36,7 +35,8 @@ constexpr int kLoopDone = 0, kLoopHandOver = 1, kLoopRestart = 2, kLoopLost = 3;
 
 constexpr int kLoopCluster = 16;    // teams of up to this many blocks are thread-block clusters
 constexpr int kLoopGrid = 148;      // blocks of the largest team, a cooperative grid (one block per SM)
-constexpr int kLoopBeads = 250000;  // larger networks run in the graph loop
+constexpr int kLoopBeads = 350000;  // larger networks run in the graph loop
+constexpr int kLoopWideBeads = 75000;  // larger ones take blocks of 512 threads
 
 // Blocks of a team for this network, 0 when the network is better off in the
 // graph loop.
@@ -46,8 +46,19 @@ int loop_team(const ChainDev& ch, const DeviceFF& ff);
 int loop_row_count(const ChainDev& ch, const DeviceFF& ff);
 size_t loop_erow_doubles(int rows);
 __host__ __device__ __forceinline__ size_t loop_vrow_doubles(int vb) { return 2 * (size_t)(vb == 1 ? 8 : vb) * 4; }
-// Kernel attributes, per device; before the first launch.
+// Kernel attributes, once per device (the current one); before the first launch.
 cudaError_t init_cg_loop();
 cudaError_t launch_cg_loop(const LoopArgs& a, int prec, int team, cudaStream_t s);
+// its parts on blocks of 512 threads (cg_loop_wide.cu)
+cudaError_t init_cg_loop_wide();
+cudaError_t launch_cg_loop_wide(const LoopArgs& a, int prec, int team, cudaStream_t s);
+
+
+// The replicas of a batch (arguments on the device; vb = 1, the order of the
+// packed batch's sums), taken in the order given, each by one cluster. bounded:
+// a call limit bounds the iterations.
+constexpr int kLoopBatchBeads = 20000;  // larger replicas run in the packed batch
+cudaError_t launch_cg_loop_batch(const LoopArgs* replicas, const int* order, int n, int* queue, int prec, bool fixed,
+                                 bool bounded, cudaStream_t s);
 
 }  // namespace mb

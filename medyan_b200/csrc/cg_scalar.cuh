@@ -4,7 +4,7 @@
 // and call limits. One thread runs it, whatever the kernels around it: the
 // graph loop's one-thread kernels and last blocks (cg.cu), the packed batch's
 // one thread per replica (cg.cu), and thread 0 of every block of the resident
-// loop (cg_loop.cu), which keeps a copy of the state per block.
+// loop (cg_loop_kernel.cuh), which keeps a copy of the state per block.
 #pragma once
 
 #include "handle.h"

@@ -203,7 +203,7 @@ struct medyan_mech {
     mb::DevBuf<double> cg_dir, cg_force2, cg_min_coords, cg_part, cg_eout;
     mb::DevBuf<mb::CGState> cg_state;
     mb::DevBuf<mb::LambdaSet> cg_lam;
-    // resident loop (cg_loop.cu): partial rows, control words; the team of the
+    // resident loop (cg_loop_kernel.cuh): partial rows, control words; the team of the
     // minimization in flight (0: the graph loop)
     mb::DevBuf<double> cg_rows;
     mb::DevBuf<int> cg_words;

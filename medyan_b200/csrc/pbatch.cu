@@ -3,6 +3,8 @@
 // own arrays (their internal bead order, their device-built neighbor lists),
 // with bead offsets shifted by each replica's base and every replica's
 // records padded to whole blocks.
+#include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "pbatch.h"
@@ -45,6 +47,7 @@ cudaError_t copy_rec(const T* src, int n, T* dst, cudaStream_t s) {
 PackedBatch::~PackedBatch() {
     if (stream) cudaStreamSynchronize(stream);
     if (graph) cudaGraphExecDestroy(graph);
+    if (pinned) cudaFreeHost(pinned);
     for (auto& sd : fork.side)
         if (sd) cudaStreamDestroy(sd);
     if (fork.fork) cudaEventDestroy(fork.fork);
@@ -53,21 +56,25 @@ PackedBatch::~PackedBatch() {
     if (stream) cudaStreamDestroy(stream);
 }
 
+medyan_status batch_streams(PackedBatch& pb) {
+    if (pb.stream) return MEDYAN_OK;
+    cudaError_t e = cudaStreamCreateWithFlags(&pb.stream, cudaStreamNonBlocking);
+    for (int k = 0; k < kForkWays && e == cudaSuccess; ++k)
+        e = cudaStreamCreateWithFlags(&pb.fork.side[k], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pb.fork.fork, cudaEventDisableTiming);
+    for (int k = 0; k < kForkWays && e == cudaSuccess; ++k)
+        e = cudaEventCreateWithFlags(&pb.fork.join[k], cudaEventDisableTiming);
+    return cuda_status(e);
+}
+
 medyan_status pack_batch(PackedBatch& pb, const std::vector<medyan_mech*>& h) {
     const int R = (int)h.size();
     long long gen = 0;
     for (auto* r : h) gen += r->ff_gen;
     if (!pb.repack && pb.R == R && pb.gen == gen && (int)pb.base.size() == R + 1) return MEDYAN_OK;
     cudaError_t e = cudaSuccess;
-    if (!pb.stream) {
-        e = cudaStreamCreateWithFlags(&pb.stream, cudaStreamNonBlocking);
-        for (int k = 0; k < kForkWays && e == cudaSuccess; ++k)
-            e = cudaStreamCreateWithFlags(&pb.fork.side[k], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&pb.fork.fork, cudaEventDisableTiming);
-        for (int k = 0; k < kForkWays && e == cudaSuccess; ++k)
-            e = cudaEventCreateWithFlags(&pb.fork.join[k], cudaEventDisableTiming);
-        if (e != cudaSuccess) return cuda_status(e);
-    }
+    const medyan_status ms = batch_streams(pb);
+    if (ms != MEDYAN_OK) return ms;
     for (auto* r : h) {
         e = cudaStreamSynchronize(r->stream);
         if (e != cudaSuccess) return cuda_status(e);
@@ -290,6 +297,148 @@ medyan_status pack_batch(PackedBatch& pb, const std::vector<medyan_mech*>& h) {
     if (e != cudaSuccess) return cuda_status(e);
     pb.gen = gen;
     pb.repack = false;
+    return MEDYAN_OK;
+}
+
+// ------------------------------------------------------------ resident loop
+bool batch_loop_takes(const std::vector<medyan_mech*>& h) {
+    for (const auto* m : h)
+        if (m->n_beads <= 0 || m->n_beads > kLoopBatchBeads || loop_team(m->chain, m->ff) == 0) return false;
+    return true;
+}
+
+medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h, const medyan_cg_params* p,
+                             double* const* coords, double* const* forces, CGState* st, double* eout, int* outcome,
+                             int* force_status) {
+    if (p->method < 0 || p->method > 2 || !(p->max_dist > 0) || !(p->lambda_max > 0) || p->line_search < 0 ||
+        p->line_search > 1)
+        return MEDYAN_ERR_INVALID_ARG;
+    const int R = (int)h.size(), kE = 2 * (MEDYAN_FF_COUNT + 1);
+    const medyan_status ms = batch_streams(pb);
+    if (ms != MEDYAN_OK) return ms;
+    int mask = -1;  // one branching mask for the batch
+    long long gen = 0;
+    for (auto* m : h) {
+        gen += m->ff_gen;
+        if (m->ff.n_branch == 0) continue;
+        if (mask < 0) mask = m->ff.branch_mask;
+        else if (mask != m->ff.branch_mask) return MEDYAN_ERR_UNSUPPORTED;
+    }
+    cudaError_t e = init_cg_loop();
+    for (auto* m : h)  // their records are complete
+        if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+    cudaStream_t s = pb.stream;
+    auto res = [&](auto& buf, size_t n) {
+        if (e == cudaSuccess) e = buf.reserve(n);
+    };
+    if (pb.loop_gen != gen || pb.loop_fixed != pb.deterministic || (int)pb.lbase.size() != R + 1) {
+        pb.loop_gen = -1;
+        pb.lbase.assign(R + 1, 0);
+        std::vector<size_t> row0(R + 1, 0);
+        const size_t vrow = loop_vrow_doubles(1);
+        for (int r = 0; r < R; ++r) {
+            pb.lbase[r + 1] = pb.lbase[r] + h[r]->n_beads;
+            row0[r + 1] = row0[r] + vrow + loop_erow_doubles(loop_row_count(h[r]->chain, h[r]->ff));
+        }
+        const size_t n3 = 3 * (size_t)pb.lbase[R];
+        for (DevBuf<double>* b : {&pb.lx, &pb.ld, &pb.lf0, &pb.lf1, &pb.lmin}) res(*b, n3);
+        res(pb.leout, (size_t)R * kE);
+        res(pb.lst, R);
+        res(pb.llam, R);
+        res(pb.loop_words, (size_t)(R + 1) * kLoopWords);  // the last words: the queue, the force status
+        res(pb.loop_rows, row0[R]);
+        if (e != cudaSuccess) return cuda_status(e);
+        std::vector<LoopArgs> args(R);
+        std::vector<int> order(R);
+        for (int r = 0; r < R; ++r) {
+            LoopArgs& a = args[r];
+            const size_t o = 3 * (size_t)pb.lbase[r];
+            a.ch = h[r]->chain;
+            a.ff = h[r]->ff;
+            a.n3 = 3 * h[r]->n_beads;
+            a.vb = 1;
+            a.fixed = pb.deterministic ? 1 : 0;
+            a.x = pb.lx.raw() + o;
+            a.d = pb.ld.raw() + o;
+            a.f0 = pb.lf0.raw() + o;
+            a.f1 = pb.lf1.raw() + o;
+            a.min_e = pb.lmin.raw() + o;
+            a.st = pb.lst.raw() + r;
+            a.lam = pb.llam.raw() + r;
+            a.eout = pb.leout.raw() + (size_t)r * kE;
+            a.vrow = pb.loop_rows.raw() + row0[r];
+            a.erow = a.vrow + vrow;
+            a.words = pb.loop_words.raw() + (size_t)r * kLoopWords;
+            a.status = pb.loop_words.raw() + (size_t)R * kLoopWords + 1;
+            order[r] = r;
+        }
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return h[a]->n_beads > h[b]->n_beads; });
+        e = pb.loop_args.assign(args.data(), R, s);
+        if (e == cudaSuccess) e = pb.loop_order.assign(order.data(), R, s);
+        if (e != cudaSuccess) return cuda_status(e);
+        pb.loop_gen = gen;
+        pb.loop_fixed = pb.deterministic;
+    }
+    // pinned staging: coordinates (in and out), forces, states, energies, words
+    const size_t n3 = 3 * (size_t)pb.lbase[R], bytes = sizeof(double) * n3;
+    const size_t need = 2 * bytes + sizeof(CGState) * R + sizeof(double) * R * kE + sizeof(int) * (R + 1) * kLoopWords;
+    if (pb.pinned_bytes < need) {
+        if (pb.pinned) cudaFreeHost(pb.pinned);
+        pb.pinned = nullptr;
+        pb.pinned_bytes = 0;
+        e = cudaMallocHost(reinterpret_cast<void**>(&pb.pinned), need);
+        if (e != cudaSuccess) return cuda_status(e);
+        pb.pinned_bytes = need;
+    }
+    double* px = reinterpret_cast<double*>(pb.pinned);
+    double* pf = px + n3;
+    double* pe = pf + n3;
+    CGState* ps = reinterpret_cast<CGState*>(pe + (size_t)R * kE);
+    int* pw = reinterpret_cast<int*>(ps + R);
+    for (int r = 0; r < R; ++r) {  // internal bead order (position q holds the caller's bead order_host[q])
+        double* to = px + 3 * (size_t)pb.lbase[r];
+        if (h[r]->identity_order) std::memcpy(to, coords[r], sizeof(double) * 3 * (size_t)h[r]->n_beads);
+        else
+            for (int q = 0; q < h[r]->n_beads; ++q)
+                std::memcpy(to + 3 * (size_t)q, coords[r] + 3 * (size_t)h[r]->order_host[q], 3 * sizeof(double));
+        ps[r] = batch_start_state(p, h[r]->n_beads);
+        ps[r].full_passes = 0;  // a cluster's pass holds its own replica's trials only
+    }
+    e = cudaMemcpyAsync(pb.lx.raw(), px, bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pb.lst.raw(), ps, sizeof(CGState) * R, cudaMemcpyHostToDevice, s);
+    for (DevBuf<double>* b : {&pb.ld, &pb.lf0, &pb.lf1})
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->raw(), 0, bytes, s);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(pb.loop_words.raw(), 0, sizeof(int) * (size_t)(R + 1) * kLoopWords, s);
+    if (e == cudaSuccess)
+        e = launch_cg_loop_batch(pb.loop_args.raw(), pb.loop_order.raw(), R,
+                                 pb.loop_words.raw() + (size_t)R * kLoopWords, h[0]->prec, pb.deterministic,
+                                 p->energy_call_limit > 0, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(px, pb.lx.raw(), bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pf, pb.lf0.raw(), bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ps, pb.lst.raw(), sizeof(CGState) * R, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(pe, pb.leout.raw(), sizeof(double) * (size_t)R * kE, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(pw, pb.loop_words.raw(), sizeof(int) * (size_t)(R + 1) * kLoopWords, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_status(e);
+    *force_status = pw[(size_t)R * kLoopWords + 1];
+    for (int r = 0; r < R; ++r) {
+        outcome[r] = pw[(size_t)r * kLoopWords + 2];
+        if (outcome[r] != kLoopDone) continue;
+        st[r] = ps[r];
+        std::memcpy(eout + (size_t)r * kE, pe + (size_t)r * kE, sizeof(double) * kE);
+        for (int out = 0; out < 2; ++out) {
+            double* to = out == 0 ? coords[r] : (forces ? forces[r] : nullptr);
+            if (!to) continue;
+            const double* from = (out == 0 ? px : pf) + 3 * (size_t)pb.lbase[r];
+            if (h[r]->identity_order) std::memcpy(to, from, sizeof(double) * 3 * (size_t)h[r]->n_beads);
+            else
+                for (int q = 0; q < h[r]->n_beads; ++q)
+                    std::memcpy(to + 3 * (size_t)h[r]->order_host[q], from + 3 * (size_t)q, 3 * sizeof(double));
+        }
+    }
     return MEDYAN_OK;
 }
 

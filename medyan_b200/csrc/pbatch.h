@@ -12,6 +12,7 @@
 
 #include <vector>
 
+#include "cg_loop.h"
 #include "handle.h"
 
 namespace mb {
@@ -72,6 +73,20 @@ struct PackedBatch {
     bool deterministic = false;
     bool graph_det = false;
 
+    // resident loop (cg_loop_kernel.cuh): a replica per cluster, on its handle's own
+    // records and these vectors; arguments, control words, sums' rows, the
+    // order of the queue, pinned staging of coordinates and forces
+    DevBuf<LoopArgs> loop_args;
+    DevBuf<int> loop_words, loop_order;
+    DevBuf<double> loop_rows, lx, ld, lf0, lf1, lmin, leout;
+    DevBuf<CGState> lst;
+    DevBuf<LambdaSet> llam;
+    std::vector<int> lbase;           // bead base of each replica (R + 1)
+    long long loop_gen = -1;          // the replicas' generations and settings of loop_args
+    bool loop_fixed = false;
+    unsigned char* pinned = nullptr;
+    size_t pinned_bytes = 0;
+
     cudaStream_t stream = nullptr;
     Fork fork{};
 
@@ -85,6 +100,19 @@ struct PackedBatch {
 
 // Builds (or rebuilds) the packed arrays from the replicas' handles.
 medyan_status pack_batch(PackedBatch& pb, const std::vector<medyan_mech*>& h);
+// The stream and side streams, made once.
+medyan_status batch_streams(PackedBatch& pb);
+// Whether the resident loop takes this batch (cg_loop_kernel.cuh), and one batched
+// minimization there: coordinates in and out of the callers' arrays, the state
+// and energies of replica r into st[r] and eout + 2 r (MEDYAN_FF_COUNT + 1).
+// outcome[r] is not kLoopDone for a replica that met a pair which needs a
+// quadrature: nothing of it is written.
+bool batch_loop_takes(const std::vector<medyan_mech*>& h);
+medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h, const medyan_cg_params* p,
+                             double* const* coords, double* const* forces, CGState* st, double* eout, int* outcome,
+                             int* force_status);
+// The start state of a replica with nb beads.
+CGState batch_start_state(const medyan_cg_params* p, int nb);
 // Runs one batched minimization on the packed arrays (coordinates already in
 // pb.x); results stay on the device (pb.x, pb.fcur, pb.st, pb.eout).
 medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p);

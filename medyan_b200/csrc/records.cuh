@@ -1,5 +1,5 @@
 // records.cuh — the per-record and per-lane work of a pass, shared by the
-// fused passes (pass.cu) and the resident minimizer loop (cg_loop.cu): one
+// fused passes (pass.cu) and the resident minimizer loop (cg_loop_kernel.cuh): one
 // lane of a chain warp tile, one generic record, one branch point. Pos maps a
 // coordinate offset to a position; each kernel brings its own (read-only
 // loads where a kernel's positions do not change, plain loads where they do).
@@ -37,7 +37,7 @@ __device__ __forceinline__ T3<R> shfl_down3(const T3<R>& v) {
 // terms acting on it to f and the link's and bend's energy to es and eb.
 template <class R, bool E, bool F, class Target>
 __device__ __forceinline__ void chain_lane(const V3& cprev, const V3& c, const V3& cnext, unsigned fl, const double2& lp,
-                                           const double2& bp, bool own, int q, const Target& t, double* f,
+                                           const double2& bp, bool own, int q, const Target& t, double* __restrict__ f,
                                            double& es, double& eb) {
     if constexpr (F) {
         T3<R> Fl{0, 0, 0}, A{0, 0, 0}, B{0, 0, 0};
@@ -65,7 +65,7 @@ __device__ __forceinline__ void chain_lane(const V3& cprev, const V3& c, const V
 // linker, 3 motor, 5 boundary): energy into acc[0], forces added to f.
 template <class R, bool E, bool F, class Target, class Pos>
 __device__ __forceinline__ void bonded_record(const DeviceFF& ff, const Target& t, const Pos& P,
-                                              double* f, int s, int i, double (&acc)[4]) {
+                                              double* __restrict__ f, int s, int i, double (&acc)[4]) {
     switch (s) {
         case 0:
             if (i < ff.n_stretch) {
@@ -132,7 +132,7 @@ __device__ __forceinline__ void bonded_record(const DeviceFF& ff, const Target& 
 
 // Branch point i: energies of its four potentials into acc, forces added to f.
 template <class R, bool E, bool F, class Target, class Pos>
-__device__ __forceinline__ void branch_record(const DeviceFF& ff, const Target& t, const Pos& P, double* f, int i,
+__device__ __forceinline__ void branch_record(const DeviceFF& ff, const Target& t, const Pos& P, double* __restrict__ f, int i,
                                               double (&acc)[4]) {
     const int4 q = ff.branch_bs[i];
     const double4 pa = ff.branch_pa[i], pb = ff.branch_pb[i];
