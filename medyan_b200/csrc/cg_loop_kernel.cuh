@@ -228,8 +228,12 @@ __device__ __forceinline__ void chain_energies(const ChainDev& ch, const Pos& P,
     V3 cp = shfl_up3(c), cn = shfl_down3(c);
     if (lane == 0) cp = ce;
     if (lane == 31) cn = ce;
-    if (fl & kLink) es += stretch_energy<double>(c, cn, lp.x, lp.y);
-    if (fl & kBend) eb += bend_energy<double>(diff<double>(cp, c), diff<double>(c, cn), bp.x, bp.y);
+    const T3<double> r = diff<double>(c, cn), r0 = diff<double>(cp, c);
+    const double len = sqrt(dot(r, r));
+    double before = __shfl_up_sync(kFull, len, 1);
+    if (lane == 0) before = sqrt(dot(r0, r0));
+    if (fl & kLink) es += stretch_energy_of(len, lp.x, lp.y);
+    if (fl & kBend) eb += bend_energy_of<double>(r0, r, before, len, bp.x, bp.y);
 }
 
 __device__ __forceinline__ double tree8(const double (*v)[kRowVals], int j) {

@@ -108,13 +108,26 @@ __global__ void __launch_bounds__(kMaxShapeThreads) k_chain_forces(const ChainDe
     }
 }
 
+// Energies of a position's link and bend at cp, c, cn (all 32 lanes call). A
+// bond's length serves its link and both its bends: one square root per lane,
+// the previous bond's from the lane before.
+__device__ __forceinline__ void chain_energies(const V3& cp, const V3& c, const V3& cn, unsigned char fl, const double2& lp,
+                                               const double2& bp, int lane, double (&acc)[2]) {
+    const T3<double> r = diff<double>(c, cn), r0 = diff<double>(cp, c);
+    const double len = sqrt(dot(r, r));
+    double before = __shfl_up_sync(kFull, len, 1);
+    if (lane == 0) before = sqrt(dot(r0, r0));
+    if (fl & kLink) acc[0] += stretch_energy_of(len, lp.x, lp.y);
+    if (fl & kBend) acc[1] += bend_energy_of<double>(r0, r, before, len, bp.x, bp.y);
+}
+
 // Energies. Each warp owns 32 consecutive positions and each lane the link
 // and bend of its own position, at up to KMAX step sizes from one read of x
 // and d (MOVE), or at x itself (a plain pass: one evaluation, copied to every
 // requested slot). A fixed grid (grid-stride over warp tiles) keeps the
 // per-block partial sums deterministic. The plain variant holds no trial
 // state, which keeps it at four blocks per SM.
-template <class R, int KMAX, bool MOVE>
+template <int KMAX, bool MOVE>
 __global__ void __launch_bounds__(kThreads, KMAX == 1 ? 4 : 2)
     k_chain_energy(const ChainDev ch, const double* __restrict__ x, const double* __restrict__ d,
                    const LambdaSet* __restrict__ lset, double* __restrict__ partial, int nblk_total, int blk_off,
@@ -157,25 +170,17 @@ __global__ void __launch_bounds__(kThreads, KMAX == 1 ? 4 : 2)
             if (lane == 0) cp = ce;
             if (lane == 31) cn = ce;
             if (!MOVE) {
-                if (fl & kLink) acc[0][0] += stretch_energy<R>(c, cn, lp.x, lp.y);
-                if (fl & kBend) acc[0][1] += bend_energy<R>(diff<R>(cp, c), diff<R>(c, cn), bp.x, bp.y);
+                chain_energies(cp, c, cn, fl, lp, bp, lane, acc[0]);
                 continue;
             }
             V3 dp = shfl_up3(dc), dn = shfl_down3(dc);
             if (lane == 0) dp = de;
             if (lane == 31) dn = de;
-            if (fl) {
     #pragma unroll
-                for (int k = 0; k < KMAX; ++k) {
-                    if (k >= K) break;
-                    const double lam = lset ? lset->lam[k] : 0.0;
-                    const V3 Pc = move3(c, lam, dc), Pn = move3(cn, lam, dn);
-                    if (fl & kLink) acc[k][0] += stretch_energy<R>(Pc, Pn, lp.x, lp.y);
-                    if (fl & kBend) {
-                        const V3 Pp = move3(cp, lam, dp);
-                        acc[k][1] += bend_energy<R>(diff<R>(Pp, Pc), diff<R>(Pc, Pn), bp.x, bp.y);
-                    }
-                }
+            for (int k = 0; k < KMAX; ++k) {
+                if (k >= K) break;
+                const double lam = lset ? lset->lam[k] : 0.0;
+                chain_energies(move3(cp, lam, dp), move3(c, lam, dc), move3(cn, lam, dn), fl, lp, bp, lane, acc[k]);
             }
         }
     #pragma unroll
@@ -251,13 +256,9 @@ void launch_chain_energy(const ChainDev& ch, int prec, const double* x, const do
     const int nrows = table ? table_blocks : chain_blocks(ch);
     if (nrows <= 0) return;
     const int g = table && nrows > kBatchGridCap ? kBatchGridCap : nrows;
-    if (prec == MEDYAN_PREC_MIXED) {
-        if (d) k_chain_energy<float, kMaxLambda, true><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
-        else k_chain_energy<float, 1, false><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
-    } else {
-        if (d) k_chain_energy<double, kMaxLambda, true><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
-        else k_chain_energy<double, 1, false><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
-    }
+    (void)prec;  // energies are FP64 in both modes
+    if (d) k_chain_energy<kMaxLambda, true><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
+    else k_chain_energy<1, false><<<g, kThreads, 0, s>>>(ch, x, d, lam, partial, nblk_total, blk_off, table, nrows);
 }
 
 void launch_to_internal(int n3, const int* order, const double* ext, double* in, cudaStream_t s) {

@@ -11,9 +11,42 @@
 
 namespace mb {
 
+// x / y for several x, given r = 1/y rounded to nearest: a quotient is refined
+// twice by its exact residual (Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: from a
+// faithful quotient one such step gives the correctly rounded one), so the
+// result is x / y bit for bit while nothing overflows or becomes subnormal,
+// and NaN where y is 0 or infinite. Five dependent operations and no branch,
+// where a division is about 140 cycles with a branch in it.
+__device__ __forceinline__ double div_by(double x, double y, double r) {
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-y, q, x), r, q);
+    return __fma_rn(__fma_rn(-y, q, x), r, q);
+}
+
+// Quotients by one denominator: in FP64 from its reciprocal, else divisions.
+// The pair formulas divide several times by each of their roots; with these
+// the FP64 force of a pair takes 14 divisions instead of 67.
+template <class R>
+struct Over {
+    R y;
+    __device__ __forceinline__ explicit Over(R d) : y(d) {}
+    __device__ __forceinline__ R operator()(R x) const { return x / y; }
+};
+template <>
+struct Over<double> {
+    double y, r;
+    __device__ __forceinline__ explicit Over(double d) {
+        y = d;
+        r = __drcp_rn(d);
+    }
+    __device__ __forceinline__ double operator()(double x) const { return div_by(x, y, r); }
+};
+
 template <class R>
 struct ExclS {
     R a, b, c, d, e, F, AA, BB, CC, DD, EE, FF, GG, HH, JJ, ATG1, ATG2, ATG3, ATG4;
+    R sum;  // CC/AA ATG1 + GG/EE ATG2 + DD/BB ATG3 + HH/FF ATG4
 };
 
 template <class R>
@@ -72,10 +105,12 @@ __device__ __forceinline__ void excl_scalars(const P3& c1, const P3& c2, const P
     R cpz = vA.x * vB.y - vA.y * vB.x;
     R JJ = cpx * vC.x + cpy * vC.y + cpz * vC.z;
     s.JJ = -JJ * JJ;
-    s.ATG1 = atan_r<R>((a + e) / s.AA) - atan_r<R>(e / s.AA);
-    s.ATG2 = atan_r<R>((a + e - d) / s.EE) - atan_r<R>((e - d) / s.EE);
-    s.ATG3 = atan_r<R>((F) / s.BB) - atan_r<R>((F - b) / s.BB);
-    s.ATG4 = atan_r<R>((d + F) / s.FF) - atan_r<R>((d + F - b) / s.FF);
+    const Over<R> oA(s.AA), oE(s.EE), oB(s.BB), oF(s.FF);
+    s.ATG1 = atan_r<R>(oA(a + e)) - atan_r<R>(oA(e));
+    s.ATG2 = atan_r<R>(oE(a + e - d)) - atan_r<R>(oE(e - d));
+    s.ATG3 = atan_r<R>(oB(F)) - atan_r<R>(oB(F - b));
+    s.ATG4 = atan_r<R>(oF(d + F)) - atan_r<R>(oF(d + F - b));
+    s.sum = oA(s.CC) * s.ATG1 + oE(s.GG) * s.ATG2 + oB(s.DD) * s.ATG3 + oF(s.HH) * s.ATG4;
 }
 
 // Analytic pair energy (:355 and :393-435). kRS = krep*L1*L2.
@@ -83,8 +118,7 @@ template <class R, class P3 = V3>
 __device__ __forceinline__ R excl_energy_r(const P3& c1, const P3& c2, const P3& c3, const P3& c4, double kRS) {
     ExclS<R> s;
     excl_scalars<R, P3>(c1, c2, c3, c4, s);
-    return R(0.5) * R(kRS) / s.JJ *
-           (s.CC / s.AA * s.ATG1 + s.GG / s.EE * s.ATG2 + s.DD / s.BB * s.ATG3 + s.HH / s.FF * s.ATG4);
+    return R(0.5) * R(kRS) / s.JJ * s.sum;
 }
 template <class R, class P3 = V3>
 __device__ __forceinline__ double excl_energy(const P3& c1, const P3& c2, const P3& c3, const P3& c4, double kRS) {
@@ -102,13 +136,15 @@ __device__ __forceinline__ bool in_plane(const V3& p1, const V3& p2, const V3& p
     double v3[3] = {p4.x - p1.x, p4.y - p1.y, p4.z - p1.z};
     double cp[3] = {v1[1] * v2[2] - v1[2] * v2[1], v1[2] * v2[0] - v1[0] * v2[2], v1[0] * v2[1] - v1[1] * v2[0]};
     double n1 = sqrt(cp[0] * cp[0] + cp[1] * cp[1] + cp[2] * cp[2]);
-    cp[0] = cp[0] / n1;
-    cp[1] = cp[1] / n1;
-    cp[2] = cp[2] / n1;
+    const Over<double> o1(n1);
+    cp[0] = o1(cp[0]);
+    cp[1] = o1(cp[1]);
+    cp[2] = o1(cp[2]);
     double n3 = sqrt(v3[0] * v3[0] + v3[1] * v3[1] + v3[2] * v3[2]);
-    v3[0] = v3[0] / n3;
-    v3[1] = v3[1] / n3;
-    v3[2] = v3[2] / n3;
+    const Over<double> o3(n3);
+    v3[0] = o3(v3[0]);
+    v3[1] = o3(v3[1]);
+    v3[2] = o3(v3[2]);
     return fabs(v3[0] * cp[0] + v3[1] * cp[1] + v3[2] * cp[2]) < 1e-1;
 }
 __device__ __forceinline__ V3 move_bead2_out_of_plane(const V3& p1, const V3& p2, const V3& p3, double d) {
@@ -116,9 +152,10 @@ __device__ __forceinline__ V3 move_bead2_out_of_plane(const V3& p1, const V3& p2
     double v2[3] = {p3.x - p1.x, p3.y - p1.y, p3.z - p1.z};
     double n[3] = {v1[1] * v2[2] - v1[2] * v2[1], v1[2] * v2[0] - v1[0] * v2[2], v1[0] * v2[1] - v1[1] * v2[0]};
     double m = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    n[0] = n[0] / m;
-    n[1] = n[1] / m;
-    n[2] = n[2] / m;
+    const Over<double> om(m);
+    n[0] = om(n[0]);
+    n[1] = om(n[1]);
+    n[2] = om(n[2]);
     return V3{p2.x + n[0] * d, p2.y + n[1] * d, p2.z + n[2] * d};
 }
 // Dual positions: the in-plane test on the values, the move on the duals.
@@ -268,7 +305,9 @@ __device__ __forceinline__ bool excl_force_exact(const P3& c1, P3 c2, const P3& 
     const R AA = S.AA, BB = S.BB, CC = S.CC, DD = S.DD, EE = S.EE, FF = S.FF, GG = S.GG, HH = S.HH;
     const R JJ = S.JJ, ATG1 = S.ATG1, ATG2 = S.ATG2, ATG3 = S.ATG3, ATG4 = S.ATG4;
     const R invJJ = R(1) / JJ;
-    const R sumBlock = CC / AA * ATG1 + GG / EE * ATG2 + DD / BB * ATG3 + HH / FF * ATG4;
+    const R sumBlock = S.sum;
+    const Over<R> oA(AA), oE(EE), oB(BB), oF(FF);
+    const Over<R> oA2(AA * AA), oE2(EE * EE), oB2(BB * BB), oF2(FF * FF);
     const R enFactor = R(kRS) * invJJ / R(2);
     const R A1 = AA * AA / (AA * AA + (a + e) * (a + e));
     const R A2 = AA * AA / (AA * AA + e * e);
@@ -278,36 +317,36 @@ __device__ __forceinline__ bool excl_force_exact(const P3& c1, P3 c2, const P3& 
     const R B2 = BB * BB / (BB * BB + (F - b) * (F - b));
     const R F1 = FF * FF / (FF * FF + (d + F) * (d + F));
     const R F2 = FF * FF / (FF * FF + (d + F - b) * (d + F - b));
-    const R bA_C = ATG1 / AA;
-    const R bA_A = -(ATG1 * CC) / (AA * AA) + (-A1 * (a + e) + A2 * e) * CC / (AA * AA * AA);
-    const R bA_e = ((A1 - A2) * CC) / (AA * AA);
-    const R bA_a = (A1 * CC) / (AA * AA);
-    const R bE_G = ATG2 / EE;
-    const R bE_E = -(ATG2 * GG) / (EE * EE) + (-E1 * (a + e - d) + E2 * (e - d)) * GG / (EE * EE * EE);
-    const R bE_emd = ((E1 - E2) * GG) / (EE * EE);
-    const R bE_a = (E1 * GG) / (EE * EE);
-    const R bB_D = ATG3 / BB;
-    const R bB_B = -(ATG3 * DD) / (BB * BB) + (-B1 * F + B2 * (F - b)) * DD / (BB * BB * BB);
-    const R bB_fmb = ((B1 - B2) * DD) / (BB * BB);
-    const R bB_b = (B1 * DD) / (BB * BB);
-    const R bF_H = ATG4 / FF;
-    const R bF_F = -(ATG4 * HH) / (FF * FF) + (-F1 * (d + F) + F2 * (d + F - b)) * HH / (FF * FF * FF);
-    const R bF_dpfmb = ((F1 - F2) * HH) / (FF * FF);
-    const R bF_b = (F1 * HH) / (FF * FF);
-    const R b11 = bA_C * (-2 * F) + bA_A * (c / AA) + bA_a * 2 + bE_G * (2 * (F - b)) + bE_E * ((b + c - 2 * F) / EE) +
-                  bE_a * 2 + bF_H * (-2 * b) + bF_F * (b / FF);
-    const R b12 = bA_C * e + bE_G * (2 * d - e) + bE_E * ((e - d) / EE) + bE_emd * (-1) + bB_D * (-F) +
-                  bF_H * (2 * d + F) + bF_F * (-(d + F) / FF) + bF_dpfmb;
-    const R b13 = bA_C * d + bA_A * (-e / AA) + bA_e + bE_G * (-d) + bE_E * (-(e - d) / EE) + bE_emd + bB_D * b +
-                  bF_H * (-b) + bF_F * (b / FF);
+    const R bA_C = oA(ATG1);
+    const R bA_A = oA2(-(ATG1 * CC)) + (-A1 * (a + e) + A2 * e) * CC / (AA * AA * AA);
+    const R bA_e = oA2((A1 - A2) * CC);
+    const R bA_a = oA2(A1 * CC);
+    const R bE_G = oE(ATG2);
+    const R bE_E = oE2(-(ATG2 * GG)) + (-E1 * (a + e - d) + E2 * (e - d)) * GG / (EE * EE * EE);
+    const R bE_emd = oE2((E1 - E2) * GG);
+    const R bE_a = oE2(E1 * GG);
+    const R bB_D = oB(ATG3);
+    const R bB_B = oB2(-(ATG3 * DD)) + (-B1 * F + B2 * (F - b)) * DD / (BB * BB * BB);
+    const R bB_fmb = oB2((B1 - B2) * DD);
+    const R bB_b = oB2(B1 * DD);
+    const R bF_H = oF(ATG4);
+    const R bF_F = oF2(-(ATG4 * HH)) + (-F1 * (d + F) + F2 * (d + F - b)) * HH / (FF * FF * FF);
+    const R bF_dpfmb = oF2((F1 - F2) * HH);
+    const R bF_b = oF2(F1 * HH);
+    const R b11 = bA_C * (-2 * F) + bA_A * oA(c) + bA_a * 2 + bE_G * (2 * (F - b)) + bE_E * oE((b + c - 2 * F)) +
+                  bE_a * 2 + bF_H * (-2 * b) + bF_F * oF(b);
+    const R b12 = bA_C * e + bE_G * (2 * d - e) + bE_E * oE((e - d)) + bE_emd * (-1) + bB_D * (-F) +
+                  bF_H * (2 * d + F) + bF_F * oF(-(d + F)) + bF_dpfmb;
+    const R b13 = bA_C * d + bA_A * oA(-e) + bA_e + bE_G * (-d) + bE_E * oE(-(e - d)) + bE_emd + bB_D * b +
+                  bF_H * (-b) + bF_F * oF(b);
     const R b21 = b12;
-    const R b22 = bE_G * (-2 * a) + bE_E * (a / EE) + bB_D * (2 * e) + bB_B * (c / BB) + bB_fmb * (-2) + bB_b * 2 +
-                  bF_H * (-2 * (a + e)) + bF_F * ((a + c + 2 * e) / FF) + bF_dpfmb * (-2) + bF_b * 2;
-    const R b23 = bA_C * (-a) + bE_G * a + bE_E * (-a / EE) + bB_D * (-d) + bB_B * (-F / BB) + bB_fmb + bF_H * d +
-                  bF_F * (-(d + F) / FF) + bF_dpfmb;
+    const R b22 = bE_G * (-2 * a) + bE_E * oE(a) + bB_D * (2 * e) + bB_B * oB(c) + bB_fmb * (-2) + bB_b * 2 +
+                  bF_H * (-2 * (a + e)) + bF_F * oF((a + c + 2 * e)) + bF_dpfmb * (-2) + bF_b * 2;
+    const R b23 = bA_C * (-a) + bE_G * a + bE_E * oE(-a) + bB_D * (-d) + bB_B * oB(-F) + bB_fmb + bF_H * d +
+                  bF_F * oF(-(d + F)) + bF_dpfmb;
     const R b31 = b13;
     const R b32 = b23;
-    const R b33 = bA_A * (a / AA) + bE_E * (a / EE) + bB_B * (b / BB) + bF_F * (b / FF);
+    const R b33 = bA_A * oA(a) + bE_E * oE(a) + bB_B * oB(b) + bF_F * oF(b);
     const R J11 = 2 * (-b * c + F * F), J12 = 2 * (c * d - e * F), J13 = 2 * (b * e - d * F);
     const R J21 = 2 * (c * d - e * F), J22 = 2 * (-a * c + e * e), J23 = 2 * (-d * e + a * F);
     const R J31 = 2 * (b * e - d * F), J32 = 2 * (-d * e + a * F), J33 = 2 * (d * d - a * b);

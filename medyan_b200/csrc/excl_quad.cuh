@@ -19,19 +19,6 @@
 
 namespace mb {
 
-// x / y for several x, given r = 1/y rounded to nearest: a quotient is refined
-// twice by its exact residual (Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: from a
-// faithful quotient one such step gives the correctly rounded one), so the
-// result is x / y bit for bit while nothing overflows or becomes subnormal,
-// and NaN where y is 0 or infinite. Five dependent operations and no branch,
-// where a division is about 140 cycles with a branch in it.
-__device__ __forceinline__ double div_by(double x, double y, double r) {
-    double q = __dmul_rn(x, r);
-    q = __fma_rn(__fma_rn(-y, q, x), r, q);
-    return __fma_rn(__fma_rn(-y, q, x), r, q);
-}
-
 struct ExclQuad {
     double a, b, c, d, e, F;      // dot products of the pair (excl_scalars)
     double JJ;                    // minus the square of the triple product

@@ -31,7 +31,7 @@
 // fallbacks round as the reference's code does).
 #include "handle.h"
 #include "records.cuh"
-#include "excl.cuh"
+#include "excl_quad.cuh"
 #include "quadrature.cuh"
 #include "pass.h"
 
@@ -103,6 +103,7 @@ constexpr int main_blocks_per_sm() {
     return kMainBlocksPerSM;
 }
 constexpr int kExclThreadsMax = 128;
+constexpr int kQuadPairs = 8000;  // pairs up to which four lanes share one (pass_geometry)
 
 // Positions of a pass: x, or x + lam*d rounded as calcCoordLineSearch.
 struct Pos {
@@ -697,44 +698,78 @@ __global__ void __launch_bounds__(kPassThreads) k_pass_branch(const __grid_const
 }
 
 // ------------------------------------------------------------ excluded volume
-// One pair per thread, FP64. A pair whose analytic energy or forces the
-// reference would reject goes to the fallback queue instead.
-template <bool E, bool F, bool EXACT>
+// FP64. A pair whose analytic energy or forces the reference would reject goes
+// to the fallback queue instead.
+template <bool E, bool F>
+__device__ __forceinline__ bool queue_pair(const PassArgs& a, int i) {
+    if constexpr (E) {
+        const int slot = atomicAdd(a.e_fb_count, 1);
+        if (slot < a.e_fb_cap) a.e_fb_list[slot] = make_int2(i, 0);
+        else atomicOr(a.e_bad, 2);
+    } else {
+        const int slot = atomicAdd(a.f_fb_count, 1);
+        if (slot < a.f_fb_cap) a.f_fb_list[slot] = i;
+        else atomicOr(a.f_status, 2);
+    }
+    return true;
+}
+
+// QUAD: four lanes per pair (excl_quad.cuh), for networks whose pairs leave the
+// GPU idle; else one pair per thread.
+template <bool E, bool F, bool EXACT, bool QUAD>
 __global__ void __launch_bounds__(kExclThreadsMax) k_pass_excl(const __grid_constant__ PassArgs a) {
     PASS_TRACE_BEGIN
+    static_assert(E != F, "energies and forces are separate passes");
     if (F && a.t.skip && *a.t.skip) return;
     double* __restrict__ f = F ? target_force(a.t) : nullptr;
     const Pos P = pos_of(a);
     const DeviceFF& ff = a.ff;
     double acc[kExclVals] = {0.0};
     bool queued = false;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ff.n_excl; i += gridDim.x * blockDim.x) {
-        const int4 q = ff.excl_bs[i];
-        const double krs = ff.excl_krs[i];
-        const V3 c1 = P(q.x), c2 = P(q.y), c3 = P(q.z), c4 = P(q.w);
-        if constexpr (E) {
-            const double U = excl_energy<double>(c1, c2, c3, c4, krs);
-            if (excl_energy_bad(U)) {
-                const int slot = atomicAdd(a.e_fb_count, 1);
-                if (slot < a.e_fb_cap) a.e_fb_list[slot] = make_int2(i, 0);
-                else atomicOr(a.e_bad, 2);
-                queued = true;
+    if constexpr (QUAD) {
+        const int j = threadIdx.x & 3, per = blockDim.x >> 2;
+        for (int i0 = blockIdx.x * per; i0 < ff.n_excl; i0 += gridDim.x * per) {
+            const int i = i0 + (threadIdx.x >> 2), ic = min(i, ff.n_excl - 1);
+            const int4 q = ff.excl_bs[ic];
+            const double krs = ff.excl_krs[ic];
+            // lane j of a pair fetches bead j and gets the force on it
+            const int o = j < 2 ? (j == 0 ? q.x : q.y) : (j == 2 ? q.z : q.w);
+            const V3 own = P(o);
+            const V3 c1 = quad_lane3(own, 0), c2 = quad_lane3(own, 1), c3 = quad_lane3(own, 2), c4 = quad_lane3(own, 3);
+            if constexpr (E) {
+                const double U = excl_energy_quad(j, c1, c2, c3, c4, krs);
+                if (i < ff.n_excl && j == 0) {
+                    if (excl_energy_bad(U)) queued = queue_pair<E, F>(a, i);
+                    else acc[0] += U;
+                }
             } else {
-                acc[0] += U;
+                T3<double> fo;
+                const bool ok = excl_force_quad<EXACT>(j, c1, c2, c3, c4, krs, fo);
+                if (i < ff.n_excl) {
+                    if (ok) target_add(a.t, f, o, fo.x, fo.y, fo.z);
+                    else if (j == 0) queued = queue_pair<E, F>(a, i);
+                }
             }
         }
-        if constexpr (F) {
-            T3<double> fo[4];
-            if (excl_force<EXACT>(c1, c2, c3, c4, krs, fo)) {
-                target_add(a.t, f, q.x, fo[0].x, fo[0].y, fo[0].z);
-                target_add(a.t, f, q.y, fo[1].x, fo[1].y, fo[1].z);
-                target_add(a.t, f, q.z, fo[2].x, fo[2].y, fo[2].z);
-                target_add(a.t, f, q.w, fo[3].x, fo[3].y, fo[3].z);
+    } else {
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ff.n_excl; i += gridDim.x * blockDim.x) {
+            const int4 q = ff.excl_bs[i];
+            const double krs = ff.excl_krs[i];
+            const V3 c1 = P(q.x), c2 = P(q.y), c3 = P(q.z), c4 = P(q.w);
+            if constexpr (E) {
+                const double U = excl_energy<double>(c1, c2, c3, c4, krs);
+                if (excl_energy_bad(U)) queued = queue_pair<E, F>(a, i);
+                else acc[0] += U;
             } else {
-                const int slot = atomicAdd(a.f_fb_count, 1);
-                if (slot < a.f_fb_cap) a.f_fb_list[slot] = i;
-                else atomicOr(a.f_status, 2);
-                queued = true;
+                T3<double> fo[4];
+                if (excl_force<EXACT>(c1, c2, c3, c4, krs, fo)) {
+                    target_add(a.t, f, q.x, fo[0].x, fo[0].y, fo[0].z);
+                    target_add(a.t, f, q.y, fo[1].x, fo[1].y, fo[1].z);
+                    target_add(a.t, f, q.z, fo[2].x, fo[2].y, fo[2].z);
+                    target_add(a.t, f, q.w, fo[3].x, fo[3].y, fo[3].z);
+                } else {
+                    queued = queue_pair<E, F>(a, i);
+                }
             }
         }
     }
@@ -761,10 +796,15 @@ void launch_kernels(const PassArgs& a, const PassGeometry& g, int prec, cudaStre
     // the excluded-volume pairs first: their FP64 chains are the longest, and
     // their blocks should be resident before the main kernel's fill the SMs
     if (g.excl_blocks > 0) {
-        if (prec == MEDYAN_PREC_FP64)
-            k_pass_excl<E, F, true><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
-        else
-            k_pass_excl<E, F, false><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
+        // an energy's form does not depend on the precision mode
+        const bool exact = E || prec == MEDYAN_PREC_FP64;
+        if (g.excl_quad) {
+            if (exact) k_pass_excl<E, F, true, true><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
+            else k_pass_excl<E, F, E, true><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
+        } else {
+            if (exact) k_pass_excl<E, F, true, false><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
+            else k_pass_excl<E, F, E, false><<<g.excl_blocks, g.excl_threads, 0, s_excl>>>(a);
+        }
     }
     if (g.chain_blocks > 0) {
         if (a.t.d)
@@ -818,7 +858,9 @@ PassGeometry pass_geometry(const ChainDev& ch, const DeviceFF& ff, bool stream) 
     const int cap = g_num_sms * kMainBlocksPerSM;
     g.main_blocks = units < 1 ? 1 : (units < cap ? units : cap);
     g.branch_blocks = (ff.n_branch + g.threads - 1) / g.threads;
-    const int eb = (ff.n_excl + g.excl_threads - 1) / g.excl_threads;
+    g.excl_quad = ff.n_excl <= kQuadPairs;
+    const int per = g.excl_quad ? g.excl_threads / 4 : g.excl_threads;
+    const int eb = (ff.n_excl + per - 1) / per;
     const int ecap = g_num_sms * 32;
     g.excl_blocks = eb < ecap ? eb : ecap;
     // a force-only pass: one unit per block, chain units of kTilesPerWarp

@@ -24,7 +24,8 @@ constexpr int kPassThreads = 256;  // threads per block of the main and branch k
 struct PassGeometry {
     int threads;        // threads per block of the main and branch kernels (= records per bonded block)
     int seg[6];         // first bonded block of leftover stretch, leftover bend, linker, motor, boundary; end
-    int excl_threads;   // pairs per excluded-volume block
+    int excl_threads;   // threads per excluded-volume block
+    bool excl_quad;     // four lanes per pair, else one
     int nch;            // chain blocks of the main kernel (threads/32 warp tiles of 30 beads each)
     int nb_main;        // bonded blocks of the main kernel (segments 0-3 and 5)
     int main_blocks, branch_blocks, excl_blocks;

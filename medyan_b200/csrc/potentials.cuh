@@ -55,6 +55,11 @@ __device__ __forceinline__ double stretch_energy(const P3& c1, const P3& c2, dou
     LenDev<R> L = length_dev<R>(c2.x - c1.x, c2.y - c1.y, c2.z - c1.z, l0);
     return double(R(0.5) * R(k) * L.dev * L.dev);
 }
+// The same from the bond length (FP64: dist - l0 is the deviation).
+__device__ __forceinline__ double stretch_energy_of(double dist, double k, double l0) {
+    const double dev = dist - l0;
+    return 0.5 * k * dev * dev;
+}
 // Force on c2 (c1 receives the negative).
 template <class R, class P3 = V3>
 __device__ __forceinline__ T3<R> stretch_force(const P3& c1, const P3& c2, double k, double l0) {
@@ -70,10 +75,9 @@ __device__ __forceinline__ T3<R> stretch_force(const P3& c1, const P3& c2, doubl
 // BranchingBendingCosine, Branching/BranchingBendingCosine.cpp:196-330.
 // r1 = p2 - p1 and r2 = p4 - p3 (filament: p3 = p2).
 // ---------------------------------------------------------------------------
+// The bond lengths L1 = |r1|, L2 = |r2| are given.
 template <class R>
-__device__ __forceinline__ double bend_energy(const T3<R>& r1, const T3<R>& r2, double k, double eqt) {
-    R L1 = sqrt(dot(r1, r1));
-    R L2 = sqrt(dot(r2, r2));
+__device__ __forceinline__ double bend_energy_of(const T3<R>& r1, const T3<R>& r2, R L1, R L2, double k, double eqt) {
     R L1L2 = L1 * L2;
     R l1l2 = dot(r1, r2);
     if (are_equal(eqt, 0.0)) {
@@ -99,6 +103,11 @@ __device__ __forceinline__ double bend_energy(const T3<R>& r1, const T3<R>& r2, 
     R sinA = stdmax<R>(sqrt(R(1) - cosA * cosA), R(0));
     R cosAmB = cosA * R(cos(eqt)) + sinA * R(sin(eqt));
     return double(R(k) * (R(1) - cosAmB));
+}
+
+template <class R>
+__device__ __forceinline__ double bend_energy(const T3<R>& r1, const T3<R>& r2, double k, double eqt) {
+    return bend_energy_of<R>(r1, r2, sqrt(dot(r1, r1)), sqrt(dot(r2, r2)), k, eqt);
 }
 
 // Returns (Fr1, Fr2): the filament bead forces are -Fr1, Fr1 - Fr2, Fr2; the

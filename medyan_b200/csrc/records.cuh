@@ -33,7 +33,7 @@ __device__ __forceinline__ T3<R> shfl_down3(const T3<R>& v) {
 }
 
 // One lane's share of a chain warp tile: the link (q, q+1) and the bend centred
-// at q are evaluated once; lanes that own their position (own) add the five
+// at q are evaluated once; lanes that own their position (own: not lane 0) add the five
 // terms acting on it to f and the link's and bend's energy to es and eb.
 template <class R, bool E, bool F, class Target>
 __device__ __forceinline__ void chain_lane(const V3& cprev, const V3& c, const V3& cnext, unsigned fl, const double2& lp,
@@ -54,9 +54,13 @@ __device__ __forceinline__ void chain_lane(const V3& cprev, const V3& c, const V
         }
     }
     if constexpr (E) {
+        // a bond's length serves its link and both its bends: one square root
+        // per lane, the previous bond's from the lane before
+        const T3<double> r = diff<double>(c, cnext);
+        const double len = sqrt(dot(r, r)), before = __shfl_up_sync(kFull, len, 1);
         if (own) {
-            if (fl & kLink) es += stretch_energy<double>(c, cnext, lp.x, lp.y);
-            if (fl & kBend) eb += bend_energy<double>(diff<double>(cprev, c), diff<double>(c, cnext), bp.x, bp.y);
+            if (fl & kLink) es += stretch_energy_of(len, lp.x, lp.y);
+            if (fl & kBend) eb += bend_energy_of<double>(diff<double>(cprev, c), r, before, len, bp.x, bp.y);
         }
     }
 }
