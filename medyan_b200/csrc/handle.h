@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -53,6 +54,11 @@ struct DevBuf {
         e = cudaMemcpyAsync(p, host, count * sizeof(T), cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return e;
         return cudaStreamSynchronize(s);
+    }
+    void swap(DevBuf& o) {
+        std::swap(p, o.p);
+        std::swap(cap, o.cap);
+        std::swap(n, o.n);
     }
     T* ptr() const { return n ? p : nullptr; }
     T* raw() const { return p; }
@@ -138,6 +144,7 @@ struct medyan_mech {
     // [0] energy, [1] forces, [2] energy then forces
     cudaGraphExec_t pass_graph[3] = {nullptr, nullptr, nullptr};
     long long pass_graph_gen[3] = {-1, -1, -1};
+    long long pass_run_gen[3] = {-1, -1, -1};  // generation the pass last ran at
     int pass_kernels[3] = {0, 0, 0};      // kernel nodes of each pass graph
 
     mb::DeviceFF ff{};
@@ -221,6 +228,7 @@ struct medyan_mech {
         double cg_energy[2 * (MEDYAN_FF_COUNT + 1)];
         int force_status;
         int cg_words[4];
+        int nl_totals[3];
     }* small = nullptr;
     int cg_graph_prec = -1;
     long long cg_graph_gen = -1;          // ff_gen the graph was captured with

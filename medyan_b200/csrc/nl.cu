@@ -170,51 +170,73 @@ __device__ __forceinline__ double dist2(const double* __restrict__ mid, int i, i
 // mode 0: count pairs per key; mode 1: write pairs (key, neighbor) for the
 // standalone build; mode 2: write excluded-volume records (branch-parent pairs
 // skipped, CylinderExclVolume.cpp:85).
+//
+// One warp per key, a lane per bin of its stencil: the bins hold a tenth of a
+// cylinder on average, so one thread per key spent its time on 27 dependent
+// loads in a row (40,000 cylinders: 48 us each for counting and writing, as
+// few blocks as the keys fill at 256 a block; now @PAIRS@ us). A key's pairs
+// stay in bin order, dx outermost, then the bin's order; when writing, keys
+// without a pair end at once.
 template <int MODE>
 __global__ void k_pairs(CylDev c, Grid G, const double* __restrict__ mid, const int* __restrict__ cell,
                         const int* __restrict__ start, const int* __restrict__ items, double rmaxsq, double rminsq,
                         int skip_branch, int* __restrict__ count, const int* __restrict__ offset,
                         int2* __restrict__ pairs, int4* __restrict__ ex_bs, double* __restrict__ ex_krs) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n || cell[i] < 0) return;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= c.n) return;
     const int ci = cell[i];
-    const int ix = ci % G.g[0], iy = (ci / G.g[0]) % G.g[1], iz = ci / (G.g[0] * G.g[1]);
-    const int idi = c.id[i], fi = c.fil[i], pi = c.pos[i];
-    int n = 0;
-    int out = MODE == 0 ? 0 : offset[i];
-    for (int dx = -1; dx <= 1; ++dx) {
-        const int jx = ix + dx;
-        if (jx < 0 || jx >= G.g[0]) continue;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int jy = iy + dy;
-            if (jy < 0 || jy >= G.g[1]) continue;
-            for (int dz = -1; dz <= 1; ++dz) {
-                const int jz = iz + dz;
-                if (jz < 0 || jz >= G.g[2]) continue;
-                const int cj = jx + G.g[0] * (jy + G.g[1] * jz);
-                for (int q = start[cj]; q < start[cj + 1]; ++q) {
-                    const int j = items[q];
-                    if (idi <= c.id[j]) continue;
-                    if (fi == c.fil[j]) {
-                        int ds = pi - c.pos[j];
-                        if ((ds < 0 ? -ds : ds) <= 2) continue;
-                    }
-                    const double d2 = dist2(mid, i, j);
-                    if (d2 > rmaxsq || d2 < rminsq) continue;
-                    if (skip_branch && c.branching[j] == i) continue;
-                    if (MODE == 1) pairs[out + n] = make_int2(i, j);
-                    if (MODE == 2) {
-                        ex_bs[out + n] = make_int4(3 * c.b1[i], 3 * c.b2[i], 3 * c.b1[j], 3 * c.b2[j]);
-                        double k = c.exclk[i];
-                        if (c.type[i] != c.type[j]) k = k < c.exclk[j] ? c.exclk[j] : k;
-                        ex_krs[out + n] = k * c.eqlen[i] * c.eqlen[j];
-                    }
-                    ++n;
-                }
-            }
-        }
+    if (ci < 0) return;
+    int out = 0;
+    if (MODE != 0) {
+        out = offset[i];
+        if (offset[i + 1] == out) return;
     }
-    if (MODE == 0) count[i] = n;
+    const int ix = ci % G.g[0], iy = (ci / G.g[0]) % G.g[1], iz = ci / (G.g[0] * G.g[1]);
+    const int jx = ix + lane / 9 - 1, jy = iy + lane / 3 % 3 - 1, jz = iz + lane % 3 - 1;
+    int q0 = 0, q1 = 0;
+    if (lane < 27 && jx >= 0 && jx < G.g[0] && jy >= 0 && jy < G.g[1] && jz >= 0 && jz < G.g[2]) {
+        const int cj = jx + G.g[0] * (jy + G.g[1] * jz);
+        q0 = start[cj];
+        q1 = start[cj + 1];
+    }
+    const int idi = c.id[i], fi = c.fil[i], pi = c.pos[i];
+    auto is_pair = [&](int j) {
+        if (idi <= c.id[j]) return false;
+        if (fi == c.fil[j]) {
+            const int ds = pi - c.pos[j];
+            if ((ds < 0 ? -ds : ds) <= 2) return false;
+        }
+        const double d2 = dist2(mid, i, j);
+        if (d2 > rmaxsq || d2 < rminsq) return false;
+        return !(skip_branch && c.branching[j] == i);
+    };
+    int n = 0;
+    for (int q = q0; q < q1; ++q) n += is_pair(items[q]) ? 1 : 0;
+    if (MODE == 0) {
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) count[i] = n;
+        return;
+    }
+    int before = n;  // pairs of the bins before this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += v;
+    }
+    out += before - n;
+    for (int q = q0; q < q1 && n > 0; ++q) {
+        const int j = items[q];
+        if (!is_pair(j)) continue;
+        if (MODE == 1) pairs[out] = make_int2(i, j);
+        if (MODE == 2) {
+            ex_bs[out] = make_int4(3 * c.b1[i], 3 * c.b2[i], 3 * c.b1[j], 3 * c.b2[j]);
+            double k = c.exclk[i];
+            if (c.type[i] != c.type[j]) k = k < c.exclk[j] ? c.exclk[j] : k;
+            ex_krs[out] = k * c.eqlen[i] * c.eqlen[j];
+        }
+        ++out;
+        --n;
+    }
 }
 
 // Canonical order for the standalone build: each key's neighbors ascending.
@@ -321,7 +343,7 @@ struct NLBuilder {
     DevBuf<double> eqlen, exclk;
     DevBuf<double> mid;
     DevBuf<int> cell, bin_count, bin_start, bin_fill, items, pair_count, pair_off, scan_sums, totals, err;
-    DevBuf<int> bcount, boff;
+    DevBuf<int> bcount, bcount_new, boff;
     DevBuf<int2> pairs;
     DevBuf<double4> planes;
     medyan_nl_params nl{};
@@ -372,8 +394,9 @@ struct NLBuilder {
         return cudaGetLastError();
     }
 
-    // Bins the midpoints and counts pairs per key; returns the pair total.
-    medyan_status count_pairs(const double* x, int skip_branch, cudaStream_t s, long long* total) {
+    // Bins the midpoints and counts pairs per key: pair_off[n] is the total,
+    // err whether a midpoint lies outside the grid. Nothing is waited for.
+    medyan_status enqueue_count(const double* x, int skip_branch, cudaStream_t s) {
         const Grid G = make_grid(nl);
         const long long nbins = (long long)G.g[0] * G.g[1] * G.g[2];
         if (nbins > (1LL << 30)) return MEDYAN_ERR_INVALID_ARG;
@@ -398,12 +421,20 @@ struct NLBuilder {
             k_scatter<<<gb, tb, 0, s>>>(n, cell.raw(), bin_start.raw(), bin_fill.raw(), items.raw());
             k_sort_bins<<<(int)((nbins + tb - 1) / tb), tb, 0, s>>>((int)nbins, bin_start.raw(), items.raw());
             const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
-            k_pairs<0><<<gb, tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
-                                         (double)rmaxsq, (double)rminsq, skip_branch, pair_count.raw(), nullptr,
-                                         nullptr, nullptr, nullptr);
+            k_pairs<0><<<key_blocks(), tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
+                                                   (double)rmaxsq, (double)rminsq, skip_branch, pair_count.raw(), nullptr,
+                                                   nullptr, nullptr, nullptr);
         }
-        e = scan(pair_count.raw(), n, pair_off.raw(), s);
-        if (e != cudaSuccess) return cuda_status(e);
+        return cuda_status(scan(pair_count.raw(), n, pair_off.raw(), s));
+    }
+
+    int key_blocks() const { return (int)((32LL * n + 255) / 256); }  // a warp per key
+
+    // The same, waited for; returns the pair total.
+    medyan_status count_pairs(const double* x, int skip_branch, cudaStream_t s, long long* total) {
+        const medyan_status st = enqueue_count(x, skip_branch, s);
+        if (st != MEDYAN_OK) return st;
+        cudaError_t e = cudaSuccess;
         int h[2] = {0, 0};
         e = cudaMemcpyAsync(&h[0], pair_off.raw() + n, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h[1], err.raw(), sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -421,31 +452,34 @@ struct NLBuilder {
         const int tb = 256, gb = (n + tb - 1) / tb;
         if (n == 0) return;
         const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
-        k_pairs<MODE><<<gb, tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
+        k_pairs<MODE><<<key_blocks(), tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
                                         (double)rmaxsq, (double)rminsq, skip_branch, nullptr, pair_off.raw(),
                                         out_pairs, ex_bs, ex_krs);
         if (MODE == 1) k_sort_pairs<<<gb, tb, 0, s>>>(n, pair_off.raw(), out_pairs);
     }
 
-    // Boundary NL + vectorization into the handle's boundary records.
-    medyan_status boundary(medyan_mech* h, const double* x, cudaStream_t s, long long* total) {
-        *total = 0;
-        if (!has_boundary || bp.n_planes <= 0) return MEDYAN_OK;
+    // Boundary NL, in two halves: counts per plane and cylinder into bcount_new
+    // (boff[n_planes n] is the total), then the handle's boundary records. The
+    // plane membership that the load forces read (bcount) changes with the
+    // second half only.
+    bool boundary_on() const { return has_boundary && bp.n_planes > 0; }
+    medyan_status enqueue_boundary_count(const double* x, cudaStream_t s) {
         const int np = bp.n_planes;
-        cudaError_t e = bcount.reserve((size_t)np * n + 1);
+        cudaError_t e = bcount_new.reserve((size_t)np * n + 1);
         if (e == cudaSuccess) e = boff.reserve((size_t)np * n + 1);
         if (e != cudaSuccess) return cuda_status(e);
         const int tb = 256, gb = (n + tb - 1) / tb;
-        if (n > 0) k_boundary_count<<<gb, tb, 0, s>>>(view(), x, planes.raw(), np, bp.cutoff, bcount.raw());
-        e = scan(bcount.raw(), np * n, boff.raw(), s);
-        if (e != cudaSuccess) return cuda_status(e);
-        int tot = 0;
-        e = cudaMemcpyAsync(&tot, boff.raw() + (size_t)np * n, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e == cudaSuccess) e = h->boundary_bs.reserve(tot);
+        if (n > 0) k_boundary_count<<<gb, tb, 0, s>>>(view(), x, planes.raw(), np, bp.cutoff, bcount_new.raw());
+        return cuda_status(scan(bcount_new.raw(), np * n, boff.raw(), s));
+    }
+    medyan_status write_boundary(medyan_mech* h, const double* x, int tot, cudaStream_t s) {
+        const int np = bp.n_planes, tb = 256, gb = (n + tb - 1) / tb;
+        cudaError_t e = h->boundary_bs.reserve(tot);
         if (e == cudaSuccess) e = h->boundary_p.reserve(tot);
         if (e == cudaSuccess) e = h->boundary_plane.reserve(tot);
-        if (e == cudaSuccess) e = h->planes.assign(planes_host4().data(), np, s);
+        if (e == cudaSuccess) e = h->planes.reserve(np);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h->planes.raw(), planes.raw(), sizeof(double4) * np, cudaMemcpyDeviceToDevice, s);
         if (e != cudaSuccess) return cuda_status(e);
         if (n > 0 && tot > 0)
             k_boundary_write<<<gb, tb, 0, s>>>(view(), x, planes.raw(), np, bp.cutoff, bp.k, bp.screen_length,
@@ -453,7 +487,7 @@ struct NLBuilder {
                                                h->boundary_plane.raw());
         h->ff.n_boundary = tot;
         h->ff.n_planes = np;
-        *total = tot;
+        bcount.swap(bcount_new);
         e = cudaGetLastError();
         boundary_built = e == cudaSuccess;
         return cuda_status(e);
@@ -565,20 +599,32 @@ medyan_status medyan_mech_rebuild_neighbors(medyan_mech* h, int64_t* n_excl_out,
     if (!h || !h->nl) return MEDYAN_ERR_INVALID_ARG;
     NLBuilder* b = reinterpret_cast<NLBuilder*>(h->nl);
     cudaStream_t s = h->stream;
-    long long total = 0;
-    medyan_status st = b->count_pairs(h->x.raw(), 1, s, &total);
+    // both lists' counts, then one wait for their totals
+    int* tot = h->small->nl_totals;  // pairs, outside the grid, boundary terms
+    tot[0] = tot[1] = tot[2] = 0;
+    medyan_status st = b->enqueue_count(h->x.raw(), 1, s);
+    if (st == MEDYAN_OK && b->boundary_on()) st = b->enqueue_boundary_count(h->x.raw(), s);
     if (st != MEDYAN_OK) return st;
-    cudaError_t e = h->excl_bs.reserve(total);
-    if (e == cudaSuccess) e = h->excl_krs.reserve(total);
+    cudaError_t e = cudaMemcpyAsync(tot, b->pair_off.raw() + b->n, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(tot + 1, b->err.raw(), sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && b->boundary_on())
+        e = cudaMemcpyAsync(tot + 2, b->boff.raw() + (size_t)b->bp.n_planes * b->n, sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_status(e);
+    if (tot[1]) return MEDYAN_ERR_OUT_OF_GRID;
+    e = h->excl_bs.reserve(tot[0]);
+    if (e == cudaSuccess) e = h->excl_krs.reserve(tot[0]);
     if (e != cudaSuccess) return cuda_status(e);
     b->write_pairs<2>(h->x.raw(), 1, nullptr, h->excl_bs.raw(), h->excl_krs.raw(), s);
-    h->ff.n_excl = (int)total;
-    long long nb = 0;
-    st = b->boundary(h, h->x.raw(), s, &nb);
-    if (st != MEDYAN_OK) return st;
+    h->ff.n_excl = tot[0];
+    const int nb = tot[2];
+    if (b->boundary_on()) {
+        st = b->write_boundary(h, h->x.raw(), nb, s);
+        if (st != MEDYAN_OK) return st;
+    }
     st = refresh_device_ff(h);
     if (st != MEDYAN_OK) return st;
-    if (n_excl_out) *n_excl_out = total;
+    if (n_excl_out) *n_excl_out = tot[0];
     if (n_boundary_out) *n_boundary_out = nb;
     return sync_status(h);
 }
