@@ -174,7 +174,7 @@ __device__ __forceinline__ double dist2(const double* __restrict__ mid, int i, i
 // One warp per key, a lane per bin of its stencil: the bins hold a tenth of a
 // cylinder on average, so one thread per key spent its time on 27 dependent
 // loads in a row (40,000 cylinders: 48 us each for counting and writing, as
-// few blocks as the keys fill at 256 a block; now @PAIRS@ us). A key's pairs
+// few blocks as the keys fill at 256 a block; now 19 and 18 us). A key's pairs
 // stay in bin order, dx outermost, then the bin's order; when writing, keys
 // without a pair end at once.
 template <int MODE>
@@ -182,7 +182,7 @@ __global__ void k_pairs(CylDev c, Grid G, const double* __restrict__ mid, const 
                         const int* __restrict__ start, const int* __restrict__ items, double rmaxsq, double rminsq,
                         int skip_branch, int* __restrict__ count, const int* __restrict__ offset,
                         int2* __restrict__ pairs, int4* __restrict__ ex_bs, double* __restrict__ ex_krs) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= c.n) return;
     const int ci = cell[i];
     if (ci < 0) return;
