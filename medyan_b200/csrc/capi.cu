@@ -372,13 +372,8 @@ static cudaError_t count_kernel_nodes(cudaGraph_t g, int* out) {
     return e;
 }
 
-// Captures and instantiates pass `which` when the force fields changed.
-cudaError_t ensure_pass_graph(medyan_mech* h, int which) {
-    if (h->pass_graph[which] && h->pass_graph_gen[which] == h->ff_gen) return cudaSuccess;
-    if (h->pass_graph[which]) cudaGraphExecDestroy(h->pass_graph[which]);
-    h->pass_graph[which] = nullptr;
-    cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return e;
+// Pass `which` at the handle's coordinates, on its streams.
+static void enqueue_pass(medyan_mech* h, int which) {
     const ForceTarget t{h->f.raw(), nullptr, nullptr, nullptr, nullptr, nullptr, h->deterministic, h->fs.status};
     if (h->pass_layout == 0 || h->pass_layout == 2)
         launch_pass_fused(h->chain, h->ff, h->prec, h->x.raw(), which == kPassEnergy ? nullptr : &t,
@@ -391,6 +386,16 @@ cudaError_t ensure_pass_graph(medyan_mech* h, int which) {
         enqueue_energy(h, h->x.raw(), nullptr, h->lam_zero.raw(), h->stream);
     else
         enqueue_forces(h, h->x.raw(), h->f.raw(), h->stream);
+}
+
+// Captures and instantiates pass `which` when the force fields changed.
+cudaError_t ensure_pass_graph(medyan_mech* h, int which) {
+    if (h->pass_graph[which] && h->pass_graph_gen[which] == h->ff_gen) return cudaSuccess;
+    if (h->pass_graph[which]) cudaGraphExecDestroy(h->pass_graph[which]);
+    h->pass_graph[which] = nullptr;
+    cudaError_t e = cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess) return e;
+    enqueue_pass(h, which);
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(h->stream, &g);
     if (e == cudaSuccess) e = count_kernel_nodes(g, &h->pass_kernels[which]);
@@ -404,8 +409,26 @@ cudaError_t ensure_pass_graph(medyan_mech* h, int which) {
     return cudaSuccess;
 }
 
+// The first pass after a vectorization goes out as stream launches, later ones
+// as the captured graph: capturing and instantiating takes 670 us, the
+// launches 40, and a caller that rebuilds its neighbor lists every step never
+// gets the graph's 5 us back. A stream the caller is capturing takes a second
+// pass as launches too: nothing can be captured apart from it then.
 cudaError_t launch_pass(medyan_mech* h, int which) {
-    cudaError_t e = ensure_pass_graph(h, which);
+    cudaError_t e;
+    if (!h->pass_graph[which] || h->pass_graph_gen[which] != h->ff_gen) {
+        cudaStreamCaptureStatus cap;
+        e = cudaStreamIsCapturing(h->stream, &cap);
+        if (e == cudaSuccess) e = cudaSetDevice(h->device);
+        if (e != cudaSuccess) return e;
+        const bool first = h->pass_run_gen[which] != h->ff_gen;
+        if (first == (cap == cudaStreamCaptureStatusNone)) {
+            h->pass_run_gen[which] = h->ff_gen;
+            enqueue_pass(h, which);
+            return cudaGetLastError();
+        }
+    }
+    e = ensure_pass_graph(h, which);
     if (e != cudaSuccess) return e;
     return cudaGraphLaunch(h->pass_graph[which], h->stream);
 }

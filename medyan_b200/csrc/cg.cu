@@ -720,7 +720,8 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     cudaStream_t s = h->stream;
     h->cg_params = *p;
     h->cg_team = loop_team(h->chain, h->ff);
-    cudaError_t e = h->cg_dir.reserve(n3 ? n3 : 1);
+    cudaError_t e = cudaSetDevice(h->device);
+    if (e == cudaSuccess) e = h->cg_dir.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess) e = h->cg_force2.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess) e = h->cg_min_coords.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess) e = h->cg_part.reserve(4 * (size_t)vec_blocks(n3) + 4);

@@ -454,7 +454,9 @@ __global__ void __launch_bounds__(kPassThreads, main_blocks_per_sm<R, E, F, LS>(
             chain_compute<R, E, F, LS>(a, P, f, w, cur, acc);
             cur = nxt;
         }
-        for (int b = blockIdx.x; b < a.nb_main; b += gridDim.x) main_chunk<R, E, F>(a, P, f, b, acc);
+        // the last blocks take the first chunks: in a small network the first
+        // blocks have the tiles
+        for (int b = gridDim.x - 1 - blockIdx.x; b < a.nb_main; b += gridDim.x) main_chunk<R, E, F>(a, P, f, b, acc);
     }
     // a force-only pass has no rows here: the main kernel's blocks take no ticket
     if constexpr (E) block_done<0, E, F>(a, acc, a.row_main + blockIdx.x, false);
@@ -942,10 +944,19 @@ void launch_pass_fused(const ChainDev& ch, const DeviceFF& ff, int prec, const d
     // streams: the force side on s, sides 0-1 (and 5 for a streamed chain);
     // the energy side on sides 2-4 (and 6) (everything on s without a fork)
     constexpr int kSides = 7;
+    bool used[kSides] = {};
     cudaStream_t sf[4] = {s, s, s, s}, se[4] = {s, s, s, s};
     if (fk) {
         cudaEventRecord(fk->fork, s);
-        for (int k = 0; k < kSides; ++k) cudaStreamWaitEvent(fk->side[k], fk->fork, 0);
+        used[0] = force && g.branch_blocks > 0;
+        used[1] = force && g.excl_blocks > 0;
+        used[2] = energy;
+        used[3] = energy && g.branch_blocks > 0;
+        used[4] = energy && g.excl_blocks > 0;
+        used[5] = force && g.chain_blocks > 0;
+        used[6] = energy && g.chain_blocks > 0;
+        for (int k = 0; k < kSides; ++k)
+            if (used[k]) cudaStreamWaitEvent(fk->side[k], fk->fork, 0);
         sf[1] = fk->side[0];
         sf[2] = fk->side[1];
         sf[3] = fk->side[5];
@@ -968,15 +979,15 @@ void launch_pass_fused(const ChainDev& ch, const DeviceFF& ff, int prec, const d
         if (n3 > 0) k_pass_zero<<<zb, kZeroThreads, 0, s>>>(*t, n3);
         if (fk) {
             cudaEventRecord(fk->mid, s);
-            cudaStreamWaitEvent(sf[1], fk->mid, 0);
-            cudaStreamWaitEvent(sf[2], fk->mid, 0);
-            cudaStreamWaitEvent(sf[3], fk->mid, 0);
+            for (int k : {0, 1, 5})
+                if (used[k]) cudaStreamWaitEvent(fk->side[k], fk->mid, 0);
         }
         if (mixed) launch_kernels<float, false, true>(a, g, prec, sf[0], sf[1], sf[2], sf[3]);
         else launch_kernels<double, false, true>(a, g, prec, sf[0], sf[1], sf[2], sf[3]);
     }
     if (fk) {
         for (int k = 0; k < kSides; ++k) {
+            if (!used[k]) continue;
             cudaEventRecord(fk->join[k], fk->side[k]);
             cudaStreamWaitEvent(s, fk->join[k], 0);
         }
