@@ -43,6 +43,17 @@ struct Over<double> {
     __device__ __forceinline__ double operator()(double x) const { return div_by(x, y, r); }
 };
 
+template <>
+struct Over<Dual> {
+    Dual y;
+    double r;
+    __device__ __forceinline__ explicit Over(const Dual& d) : y(d) { r = __drcp_rn(d.v); }
+    __device__ __forceinline__ Dual operator()(const Dual& x) const {
+        const double q = div_by(x.v, y.v, r);
+        return Dual(q, div_by(x.d - q * y.d, y.v, r));
+    }
+};
+
 template <class R>
 struct ExclS {
     R a, b, c, d, e, F, AA, BB, CC, DD, EE, FF, GG, HH, JJ, ATG1, ATG2, ATG3, ATG4;
@@ -167,7 +178,8 @@ __device__ __forceinline__ DV3 move_bead2_out_of_plane(const DV3& p1, const DV3&
     const DV3 v1 = diff<Dual>(p1, p2), v2 = diff<Dual>(p1, p3);
     DV3 n{v1.y * v2.z - v1.z * v2.y, v1.z * v2.x - v1.x * v2.z, v1.x * v2.y - v1.y * v2.x};
     const Dual m = sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
-    n = DV3{n.x / m, n.y / m, n.z / m};
+    const Over<Dual> om(m);
+    n = DV3{om(n.x), om(n.y), om(n.z)};
     return DV3{p2.x + n.x * d, p2.y + n.y * d, p2.z + n.z * d};
 }
 
