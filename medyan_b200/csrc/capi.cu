@@ -356,6 +356,133 @@ cudaError_t coords_to_host(medyan_mech* h, const double* dev, double* host, cuda
     return e;
 }
 
+// Host coordinates and results of one synchronous call through the handle's
+// pinned staging, which kernels read and write over the bus, in pieces: the
+// host copies a piece while the device moves the one before. A pageable copy is
+// staged by the driver, the call waits for it, and each small copy is an engine
+// operation of its own: an evaluation was four copies, a memset and two waits
+// around a pass of 10 us. Pinned memory takes over 1 ms to allocate from about
+// 2 MB on, so the staging is four pieces whatever the network's size. Evaluations
+// before and now: 550 beads 67 and 40 us, 10,500 142 and 76, 42,000 337 and
+// 212, 420,000 2,265 and 1,850.
+constexpr int kIoThreads = 256;
+constexpr int kIoBeads = 5460;  // beads a piece: 128 KB
+
+__global__ void k_hand_in(int n3, const double* __restrict__ host, double* __restrict__ dev) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n3) dev[i] = host[i];
+}
+// The last piece also hands out n_e energies and the status, which it clears.
+__global__ void k_hand_out(int n3, const double* __restrict__ dev, double* __restrict__ host, int n_e,
+                           const double* __restrict__ e, double* __restrict__ e_host, int* __restrict__ status,
+                           int* __restrict__ status_host) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n3) host[i] = dev[i];
+    if (i < n_e) e_host[i] = e[i];
+    if (i == 0 && status) {
+        *status_host = *status;
+        *status = 0;
+    }
+}
+
+// Whether a copy to or from host goes through the staging, which the first such
+// call makes. Memory that CUDA knows (pinned, managed) takes plain copies, which
+// need no host time there, as does everything when no staging is to be had.
+bool staged(medyan_mech* h, const double* host) {
+    cudaPointerAttributes a;
+    if (h->n_beads == 0 || cudaSetDevice(h->device) != cudaSuccess ||
+        cudaPointerGetAttributes(&a, host) != cudaSuccess || a.type != cudaMemoryTypeUnregistered)
+        return false;
+    if (h->io) return true;
+    const int slots = h->n_beads > kIoBeads ? kIoSlots : 1;
+    const int beads = h->n_beads < kIoBeads ? h->n_beads : kIoBeads;
+    cudaError_t e = cudaSuccess;
+    for (cudaEvent_t& ev : h->io_done)
+        if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+        e = cudaMallocHost(reinterpret_cast<void**>(&h->io), sizeof(double) * 3 * (size_t)beads * slots);
+    if (e != cudaSuccess) {
+        h->io = nullptr;
+        cudaGetLastError();
+    }
+    return e == cudaSuccess;
+}
+
+// Piece k: its first bead and number of beads. The copies between the caller's
+// bead order and the internal one are the host's.
+struct IoPiece {
+    int first, beads;
+    double* slot;
+    IoPiece(const medyan_mech* h, int k)
+        : first(k * kIoBeads),
+          beads(h->n_beads - first < kIoBeads ? h->n_beads - first : kIoBeads),
+          slot(h->io + 3 * (size_t)kIoBeads * (k % kIoSlots)) {}
+    int blocks() const { return (3 * beads + kIoThreads - 1) / kIoThreads; }
+    size_t bytes() const { return 3 * sizeof(double) * (size_t)beads; }
+};
+
+cudaError_t staged_in(medyan_mech* h, const double* host, double* dev) {
+    const int pieces = (h->n_beads - 1) / kIoBeads + 1;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
+        const IoPiece q(h, k);
+        if (k >= kIoSlots) e = cudaEventSynchronize(h->io_done[k % kIoSlots]);
+        if (e != cudaSuccess) break;
+        if (h->identity_order) std::memcpy(q.slot, host + 3 * (size_t)q.first, q.bytes());
+        else
+            for (int p = 0; p < q.beads; ++p)
+                std::memcpy(q.slot + 3 * p, host + 3 * (size_t)h->order_host[q.first + p], 3 * sizeof(double));
+        k_hand_in<<<q.blocks(), kIoThreads, 0, h->stream>>>(3 * q.beads, q.slot, dev + 3 * (size_t)q.first);
+        e = cudaGetLastError();
+        if (e == cudaSuccess && k + kIoSlots < pieces) e = cudaEventRecord(h->io_done[k % kIoSlots], h->stream);
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(h->stream);  // the staging is the next call's
+    return e;
+}
+
+cudaError_t staged_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status) {
+    const int pieces = (h->n_beads - 1) / kIoBeads + 1;
+    auto send = [&](int k) {
+        const IoPiece q(h, k);
+        const bool last = k == pieces - 1;
+        k_hand_out<<<q.blocks(), kIoThreads, 0, h->stream>>>(
+            3 * q.beads, dev + 3 * (size_t)q.first, q.slot, last && energies ? MEDYAN_FF_COUNT + 1 : 0,
+            h->energy_out.raw(), h->small->energy, last ? h->force_status.raw() : nullptr, &h->small->force_status);
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess && !last ? cudaEventRecord(h->io_done[k % kIoSlots], h->stream) : e;
+    };
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < pieces && k < kIoSlots && e == cudaSuccess; ++k) e = send(k);
+    for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
+        const IoPiece q(h, k);
+        e = k < pieces - 1 ? cudaEventSynchronize(h->io_done[k % kIoSlots]) : cudaStreamSynchronize(h->stream);
+        if (e != cudaSuccess) break;
+        if (h->identity_order) std::memcpy(host + 3 * (size_t)q.first, q.slot, q.bytes());
+        else
+            for (int p = 0; p < q.beads; ++p)
+                std::memcpy(host + 3 * (size_t)h->order_host[q.first + p], q.slot + 3 * p, 3 * sizeof(double));
+        if (k + kIoSlots < pieces) e = send(k + kIoSlots);
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(h->stream);
+    *status = h->small->force_status;
+    return e;
+}
+
+// The same by plain copies.
+cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status) {
+    cudaStream_t s = h->stream;
+    cudaError_t e = cudaSuccess;
+    if (energies)
+        e = cudaMemcpyAsync(h->small->energy, h->energy_out.ptr(), sizeof h->small->energy, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = coords_to_host(h, dev, host, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(&h->small->force_status, h->force_status.ptr(), sizeof(int), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->force_status.ptr(), 0, sizeof(int), s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    *status = h->small->force_status;
+    return e;
+}
+
 static cudaError_t count_kernel_nodes(cudaGraph_t g, int* out) {
     size_t n = 0;
     cudaError_t e = cudaGraphGetNodes(g, nullptr, &n);
@@ -491,6 +618,9 @@ medyan_mech::~medyan_mech() {
     if (cg_graph) cudaGraphExecDestroy(cg_graph);
     if (cg_pinned) cudaFreeHost(cg_pinned);
     if (small) cudaFreeHost(small);
+    if (io) cudaFreeHost(io);
+    for (auto& ev : io_done)
+        if (ev) cudaEventDestroy(ev);
     for (auto& g : pass_graph)
         if (g) cudaGraphExecDestroy(g);
     destroy_async(this);
@@ -577,7 +707,7 @@ medyan_status medyan_mech_destroy(medyan_mech* h) {
 
 medyan_status medyan_mech_set_coords(medyan_mech* h, const double* coord) {
     if (!h || (!coord && h->n_beads)) return MEDYAN_ERR_INVALID_ARG;
-    cudaError_t e = coords_to_device(h, coord, h->x.raw(), h->stream);
+    cudaError_t e = staged(h, coord) ? staged_in(h, coord, h->x.raw()) : coords_to_device(h, coord, h->x.raw(), h->stream);
     if (e != cudaSuccess) return cuda_status(e);
     return sync_status(h);
 }
@@ -608,15 +738,11 @@ medyan_status medyan_mech_forces(medyan_mech* h, double* force_out) {
     if (!h || (!force_out && h->n_beads)) return MEDYAN_ERR_INVALID_ARG;
     cudaError_t e = launch_pass(h, kPassForces);
     if (e != cudaSuccess) return cuda_status(e);
-    e = coords_to_host(h, h->f.raw(), force_out, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&h->small->force_status, h->force_status.ptr(), sizeof(int), cudaMemcpyDeviceToHost,
-                            h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->force_status.ptr(), 0, sizeof(int), h->stream);
+    int status = 0;
+    if (staged(h, force_out)) e = staged_out(h, h->f.raw(), force_out, false, &status);
+    else e = plain_out(h, h->f.raw(), force_out, false, &status);
     if (e != cudaSuccess) return cuda_status(e);
-    medyan_status st = sync_status(h);
-    if (st != MEDYAN_OK) return st;
-    return h->small->force_status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
+    return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
 }
 
 medyan_status medyan_mech_enqueue_energy(medyan_mech* h) {
@@ -677,23 +803,22 @@ medyan_status medyan_mech_device_buffers(medyan_mech* h, double** coord, double*
 medyan_status medyan_mech_evaluate(medyan_mech* h, const double* coord, double* e_total, double* e_per_ff,
                                    double* force_out) {
     if (!h || !coord || !e_total || !force_out) return MEDYAN_ERR_INVALID_ARG;
-    cudaError_t e = coords_to_device(h, coord, h->x.raw(), h->stream);
+    const bool in = staged(h, coord);
+    cudaError_t e = in ? staged_in(h, coord, h->x.raw()) : coords_to_device(h, coord, h->x.raw(), h->stream);
     if (e != cudaSuccess) return cuda_status(e);
     e = launch_pass(h, kPassBoth);
+    if (e != cudaSuccess) {
+        if (in) cudaStreamSynchronize(h->stream);  // the staging is the next call's
+        return cuda_status(e);
+    }
+    int status = 0;
+    e = staged(h, force_out) ? staged_out(h, h->f.raw(), force_out, true, &status)
+                             : plain_out(h, h->f.raw(), force_out, true, &status);
     if (e != cudaSuccess) return cuda_status(e);
-    double* out = h->small->energy;
-    e = cudaMemcpyAsync(out, h->energy_out.ptr(), sizeof h->small->energy, cudaMemcpyDeviceToHost, h->stream);
-    if (e == cudaSuccess) e = coords_to_host(h, h->f.raw(), force_out, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&h->small->force_status, h->force_status.ptr(), sizeof(int), cudaMemcpyDeviceToHost,
-                            h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(h->force_status.ptr(), 0, sizeof(int), h->stream);
-    if (e != cudaSuccess) return cuda_status(e);
-    medyan_status st = sync_status(h);
-    if (st != MEDYAN_OK) return st;
+    const double* out = h->small->energy;
     *e_total = out[MEDYAN_FF_COUNT];
     if (e_per_ff) std::memcpy(e_per_ff, out, sizeof(double) * MEDYAN_FF_COUNT);
-    if (h->small->force_status) return MEDYAN_ERR_NONFINITE;
+    if (status) return MEDYAN_ERR_NONFINITE;
     if (std::isinf(out[MEDYAN_FF_COUNT])) return MEDYAN_ERR_NONFINITE;
     return MEDYAN_OK;
 }

@@ -349,7 +349,8 @@ int blocks_for(int n) {
 cudaError_t upload_direction(medyan_mech* h, const double* v) {
     const int n3 = 3 * h->n_beads;
     cudaError_t e = h->hv_v.reserve(n3 ? n3 : 1);
-    if (e == cudaSuccess) e = coords_to_device(h, v, h->hv_v.raw(), h->stream);
+    if (e == cudaSuccess)
+        e = staged(h, v) ? staged_in(h, v, h->hv_v.raw()) : coords_to_device(h, v, h->hv_v.raw(), h->stream);
     return e;
 }
 
@@ -444,11 +445,8 @@ extern "C" medyan_status medyan_mech_hvp(medyan_mech* h, const double* v, double
     }
     ce = cudaGetLastError();
     int status = 0;
-    if (ce == cudaSuccess) ce = coords_to_host(h, out, hv, s);
     if (ce == cudaSuccess)
-        ce = cudaMemcpyAsync(&status, h->force_status.raw(), sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(h->force_status.raw(), 0, sizeof(int), s);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+        ce = staged(h, hv) ? staged_out(h, out, hv, false, &status) : plain_out(h, out, hv, false, &status);
     if (ce != cudaSuccess) return cuda_status(ce);
     return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
 }

@@ -18,6 +18,7 @@
 namespace mb {
 
 struct medyan_async;  // async.cu
+constexpr int kIoSlots = 4;  // pieces of the staging of host coordinates
 
 template <class T>
 struct DevBuf {
@@ -230,6 +231,10 @@ struct medyan_mech {
         int cg_words[4];
         int nl_totals[3];
     }* small = nullptr;
+    // pinned staging of the synchronous calls' coordinates and results in
+    // pieces (staged_in/staged_out), made by the first call that uses it
+    double* io = nullptr;
+    cudaEvent_t io_done[mb::kIoSlots] = {};
     int cg_graph_prec = -1;
     long long cg_graph_gen = -1;          // ff_gen the graph was captured with
     long long ff_gen = 0;                 // bumped whenever DeviceFF changes
@@ -267,6 +272,13 @@ cudaError_t launch_pass(medyan_mech* h, int which);
 // Host coordinates/forces (caller's bead order) to and from internal device
 // arrays; stream-ordered on s (the host buffer must stay valid until s syncs).
 cudaError_t coords_to_device(medyan_mech* h, const double* host, double* dev, cudaStream_t s);
+// The same through the handle's pinned staging, where staged(h, host) says
+// so, and the way out by plain copies; both ways out wait for the handle's
+// stream and hand out its force status.
+bool staged(medyan_mech* h, const double* host);
+cudaError_t staged_in(medyan_mech* h, const double* host, double* dev);
+cudaError_t staged_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
+cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
 // A minimization in two halves (cg.cu): enqueue everything on the handle's
 // stream without waiting, then wait and copy the results out.
 medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double* coord_in);

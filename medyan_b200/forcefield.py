@@ -110,14 +110,18 @@ class ForceFieldManager:
     def compute_forces(self, coord=None) -> np.ndarray:
         if coord is not None:
             self.set_coords(coord)
-        f = np.zeros(3 * self.n_beads)
+        f = np.empty(3 * self.n_beads)
         L.check(self.lib.medyan_mech_forces(self.handle, _dp(f)), "medyan_mech_forces")
         return f
+
+    def _out_like(self, x):
+        # filled by the call: not worth zeroing, except what it does not reach
+        return np.empty_like(x) if x.size == 3 * self.n_beads else np.zeros_like(x)
 
     def evaluate(self, coord):
         """Energy, per-force-field energies and forces at coord in one call."""
         x = f64(coord)
-        f = np.zeros_like(x)
+        f = self._out_like(x)
         tot = C.c_double(0.0)
         per = np.zeros(FF_COUNT)
         st = self.lib.medyan_mech_evaluate(self.handle, _dp(x), C.byref(tot), _dp(per), _dp(f))
@@ -174,7 +178,7 @@ class ForceFieldManager:
     def hvp(self, v) -> np.ndarray:
         """Hessian of the total energy at the current coordinates times v."""
         vv = f64(v)
-        hv = np.zeros_like(vv)
+        hv = self._out_like(vv)
         st = self.lib.medyan_mech_hvp(self.handle, _dp(vv), _dp(hv))
         if st not in (0, 3):
             L.check(st, "medyan_mech_hvp")
