@@ -394,7 +394,7 @@ bool staged(medyan_mech* h, const double* host) {
         cudaPointerGetAttributes(&a, host) != cudaSuccess || a.type != cudaMemoryTypeUnregistered)
         return false;
     if (h->io) return true;
-    const int slots = h->n_beads > kIoBeads ? kIoSlots : 1;
+    const int slots = h->n_beads > kIoBeads ? kIoSlots : 2;  // two arrays go out together
     const int beads = h->n_beads < kIoBeads ? h->n_beads : kIoBeads;
     cudaError_t e = cudaSuccess;
     for (cudaEvent_t& ev : h->io_done)
@@ -408,15 +408,15 @@ bool staged(medyan_mech* h, const double* host) {
     return e == cudaSuccess;
 }
 
-// Piece k: its first bead and number of beads. The copies between the caller's
+// Piece k in slot s: its first bead and number of beads. The copies between the caller's
 // bead order and the internal one are the host's.
 struct IoPiece {
     int first, beads;
     double* slot;
-    IoPiece(const medyan_mech* h, int k)
+    IoPiece(const medyan_mech* h, int k, int s)
         : first(k * kIoBeads),
           beads(h->n_beads - first < kIoBeads ? h->n_beads - first : kIoBeads),
-          slot(h->io + 3 * (size_t)kIoBeads * (k % kIoSlots)) {}
+          slot(h->io + 3 * (size_t)(h->n_beads < kIoBeads ? h->n_beads : kIoBeads) * (s % kIoSlots)) {}
     int blocks() const { return (3 * beads + kIoThreads - 1) / kIoThreads; }
     size_t bytes() const { return 3 * sizeof(double) * (size_t)beads; }
 };
@@ -425,7 +425,7 @@ cudaError_t staged_in(medyan_mech* h, const double* host, double* dev) {
     const int pieces = (h->n_beads - 1) / kIoBeads + 1;
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
-        const IoPiece q(h, k);
+        const IoPiece q(h, k, k);
         if (k >= kIoSlots) e = cudaEventSynchronize(h->io_done[k % kIoSlots]);
         if (e != cudaSuccess) break;
         if (h->identity_order) std::memcpy(q.slot, host + 3 * (size_t)q.first, q.bytes());
@@ -440,21 +440,23 @@ cudaError_t staged_in(medyan_mech* h, const double* host, double* dev) {
     return e;
 }
 
-cudaError_t staged_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status) {
-    const int pieces = (h->n_beads - 1) / kIoBeads + 1;
+cudaError_t staged_out(medyan_mech* h, const HostCopy* c, int n, bool energies, int* status) {
+    const int per = (h->n_beads - 1) / kIoBeads + 1, pieces = n * per;
     auto send = [&](int k) {
-        const IoPiece q(h, k);
+        const IoPiece q(h, k % per, k);
         const bool last = k == pieces - 1;
         k_hand_out<<<q.blocks(), kIoThreads, 0, h->stream>>>(
-            3 * q.beads, dev + 3 * (size_t)q.first, q.slot, last && energies ? MEDYAN_FF_COUNT + 1 : 0,
-            h->energy_out.raw(), h->small->energy, last ? h->force_status.raw() : nullptr, &h->small->force_status);
+            3 * q.beads, c[k / per].dev + 3 * (size_t)q.first, q.slot, last && energies ? MEDYAN_FF_COUNT + 1 : 0,
+            h->energy_out.raw(), h->small->energy, last && status ? h->force_status.raw() : nullptr,
+            &h->small->force_status);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess && !last ? cudaEventRecord(h->io_done[k % kIoSlots], h->stream) : e;
     };
     cudaError_t e = cudaSuccess;
     for (int k = 0; k < pieces && k < kIoSlots && e == cudaSuccess; ++k) e = send(k);
     for (int k = 0; k < pieces && e == cudaSuccess; ++k) {
-        const IoPiece q(h, k);
+        const IoPiece q(h, k % per, k);
+        double* host = c[k / per].host;
         e = k < pieces - 1 ? cudaEventSynchronize(h->io_done[k % kIoSlots]) : cudaStreamSynchronize(h->stream);
         if (e != cudaSuccess) break;
         if (h->identity_order) std::memcpy(host + 3 * (size_t)q.first, q.slot, q.bytes());
@@ -464,7 +466,7 @@ cudaError_t staged_out(medyan_mech* h, const double* dev, double* host, bool ene
         if (k + kIoSlots < pieces) e = send(k + kIoSlots);
     }
     if (e != cudaSuccess) cudaStreamSynchronize(h->stream);
-    *status = h->small->force_status;
+    if (status) *status = h->small->force_status;
     return e;
 }
 
@@ -616,7 +618,6 @@ medyan_mech::~medyan_mech() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
     if (cg_graph) cudaGraphExecDestroy(cg_graph);
-    if (cg_pinned) cudaFreeHost(cg_pinned);
     if (small) cudaFreeHost(small);
     if (io) cudaFreeHost(io);
     for (auto& ev : io_done)
@@ -739,7 +740,8 @@ medyan_status medyan_mech_forces(medyan_mech* h, double* force_out) {
     cudaError_t e = launch_pass(h, kPassForces);
     if (e != cudaSuccess) return cuda_status(e);
     int status = 0;
-    if (staged(h, force_out)) e = staged_out(h, h->f.raw(), force_out, false, &status);
+    const HostCopy to{h->f.raw(), force_out};
+    if (staged(h, force_out)) e = staged_out(h, &to, 1, false, &status);
     else e = plain_out(h, h->f.raw(), force_out, false, &status);
     if (e != cudaSuccess) return cuda_status(e);
     return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
@@ -812,7 +814,8 @@ medyan_status medyan_mech_evaluate(medyan_mech* h, const double* coord, double* 
         return cuda_status(e);
     }
     int status = 0;
-    e = staged(h, force_out) ? staged_out(h, h->f.raw(), force_out, true, &status)
+    const HostCopy to{h->f.raw(), force_out};
+    e = staged(h, force_out) ? staged_out(h, &to, 1, true, &status)
                              : plain_out(h, h->f.raw(), force_out, true, &status);
     if (e != cudaSuccess) return cuda_status(e);
     const double* out = h->small->energy;

@@ -617,12 +617,13 @@ using namespace mb;
 
 namespace mb {
 
-// Inputs of a minimization on the device: coordinates, state, zeroed vectors.
-static cudaError_t cg_upload(medyan_mech* h, const CGLaunch& c, cudaStream_t s) {
+// Start of a minimization from the coordinates on the device: its state, zeroed
+// vectors.
+static cudaError_t cg_start(medyan_mech* h, const CGLaunch& c, cudaStream_t s) {
     const size_t bytes = sizeof(double) * (size_t)c.n3;
     const medyan_cg_params* p = &h->cg_params;
-    CGState* ps = reinterpret_cast<CGState*>(h->cg_pinned + 2 * bytes);
-    LambdaSet* pl = reinterpret_cast<LambdaSet*>(h->cg_pinned + 2 * bytes + sizeof(CGState));
+    CGState* ps = &h->small->cg_state;
+    LambdaSet* pl = &h->small->cg_lam;
     CGState s0{};
     s0.method = p->method;
     s0.try_to_recover = p->try_to_recover;
@@ -645,8 +646,7 @@ static cudaError_t cg_upload(medyan_mech* h, const CGLaunch& c, cudaStream_t s) 
     s0.move_kind = 0;
     *ps = s0;
     *pl = LambdaSet{};
-    cudaError_t e = coords_to_device(h, reinterpret_cast<double*>(h->cg_pinned), c.x, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(c.st, ps, sizeof *ps, cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaMemcpyAsync(c.st, ps, sizeof *ps, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(c.L, pl, sizeof *pl, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(c.d, 0, bytes ? bytes : 8, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(c.f0, 0, bytes ? bytes : 8, s);
@@ -709,8 +709,8 @@ static LoopArgs loop_args(medyan_mech* h, const CGLaunch& c) {
     return a;
 }
 
-// Enqueues a whole minimization on the handle's stream. No host
-// synchronization; cg_collect reads the results.
+// Enqueues a whole minimization on the handle's stream; cg_collect reads the
+// results.
 medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double* coord_in) {
     if (!h || !p || !coord_in) return MEDYAN_ERR_INVALID_ARG;
     if (p->method < 0 || p->method > 2 || !(p->max_dist > 0) || !(p->lambda_max > 0) || p->line_search < 0 ||
@@ -733,20 +733,9 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     if (e == cudaSuccess && h->cg_team > 0) e = h->cg_words.reserve(kLoopWords);
     if (e == cudaSuccess && h->cg_team > 0) e = init_cg_loop();
     if (e != cudaSuccess) return cuda_status(e);
-    const size_t bytes = sizeof(double) * (size_t)n3;
-    // pinned staging: coordinates in, coordinates and forces out, state, lambda set
-    const size_t need = 2 * bytes + sizeof(CGState) + sizeof(LambdaSet) + 64;
-    if (h->cg_pinned_bytes < need) {
-        if (h->cg_pinned) cudaFreeHost(h->cg_pinned);
-        h->cg_pinned = nullptr;
-        h->cg_pinned_bytes = 0;
-        e = cudaMallocHost(reinterpret_cast<void**>(&h->cg_pinned), need);
-        if (e != cudaSuccess) return cuda_status(e);
-        h->cg_pinned_bytes = need;
-    }
     const CGLaunch c = make_launch(h);
-    if (n3) std::memcpy(h->cg_pinned, coord_in, bytes);
-    e = cg_upload(h, c, s);
+    e = staged(h, coord_in) ? staged_in(h, coord_in, c.x) : coords_to_device(h, coord_in, c.x, s);
+    if (e == cudaSuccess) e = cg_start(h, c, s);
     if (e == cudaSuccess && h->cg_team > 0) {
         e = cudaMemsetAsync(h->cg_words.raw(), 0, sizeof(int) * kLoopWords, s);
         if (e == cudaSuccess) e = launch_cg_loop(loop_args(h, c), h->prec, h->cg_team, s);
@@ -760,10 +749,6 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
 // stopped in front of a quadrature is finished by the graph loop first.
 medyan_status cg_collect(medyan_mech* h, double* coord_out, double* force_out, medyan_min_result* out) {
     cudaStream_t s = h->stream;
-    const size_t bytes = sizeof(double) * 3 * (size_t)h->n_beads;
-    double* px = reinterpret_cast<double*>(h->cg_pinned);
-    double* pf = reinterpret_cast<double*>(h->cg_pinned + bytes);
-    CGState* ps = reinterpret_cast<CGState*>(h->cg_pinned + 2 * bytes);
     if (h->cg_team > 0) {
         int* w = h->small->cg_words;
         cudaError_t e = cudaMemcpyAsync(w, h->cg_words.raw(), sizeof(int) * kLoopWords, cudaMemcpyDeviceToHost, s);
@@ -772,25 +757,30 @@ medyan_status cg_collect(medyan_mech* h, double* coord_out, double* force_out, m
         if (w[2] == kLoopLost) return cuda_status(cudaErrorLaunchTimeout);
         const CGLaunch c = make_launch(h);
         if (w[2] == kLoopRestart) {
-            e = cg_upload(h, c, s);  // the staged coordinates are still the caller's
+            e = cg_start(h, c, s);  // the coordinates are still the caller's
             if (e == cudaSuccess) e = cg_graph_run(h, c, s);
         } else if (w[2] == kLoopHandOver) {
             e = cg_graph_loop(h, c, s);
         }
         if (e != cudaSuccess) return cuda_status(e);
     }
-    cudaError_t e = coords_to_host(h, h->x.raw(), px, s);
-    if (e == cudaSuccess && force_out) e = coords_to_host(h, h->f.raw(), pf, s);
-    if (e != cudaSuccess) return cuda_status(e);
     double* eo = h->small->cg_energy;
-    e = cudaMemcpyAsync(ps, h->cg_state.raw(), sizeof(CGState), cudaMemcpyDeviceToHost, s);
+    cudaError_t e =
+        cudaMemcpyAsync(&h->small->cg_state, h->cg_state.raw(), sizeof(CGState), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(eo, h->cg_eout.raw(), sizeof h->small->cg_energy, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const HostCopy to[2] = {{h->x.raw(), coord_out}, {h->f.raw(), force_out}};
+    const int n = force_out ? 2 : 1;
+    bool by_stage = true;
+    for (int i = 0; i < n; ++i) by_stage = by_stage && staged(h, to[i].host);
+    if (by_stage) {
+        if (e == cudaSuccess) e = staged_out(h, to, n, false, nullptr);
+    } else {
+        for (int i = 0; i < n && e == cudaSuccess; ++i) e = coords_to_host(h, to[i].dev, to[i].host, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
     if (e != cudaSuccess) return cuda_status(e);
-    const CGState sf = *ps;
-    if (bytes) std::memcpy(coord_out, px, bytes);
-    if (force_out && bytes) std::memcpy(force_out, pf, bytes);
+    const CGState sf = h->small->cg_state;
     if (out) {
         std::memset(out, 0, sizeof *out);
         for (int i = 0; i < MEDYAN_FF_COUNT; ++i) {

@@ -445,8 +445,9 @@ extern "C" medyan_status medyan_mech_hvp(medyan_mech* h, const double* v, double
     }
     ce = cudaGetLastError();
     int status = 0;
+    const HostCopy to{out, hv};
     if (ce == cudaSuccess)
-        ce = staged(h, hv) ? staged_out(h, out, hv, false, &status) : plain_out(h, out, hv, false, &status);
+        ce = staged(h, hv) ? staged_out(h, &to, 1, false, &status) : plain_out(h, out, hv, false, &status);
     if (ce != cudaSuccess) return cuda_status(ce);
     return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
 }

@@ -218,15 +218,13 @@ struct medyan_mech {
     int cg_team = 0;
     medyan_cg_params cg_params{};
     cudaGraphExec_t cg_graph = nullptr;   // instantiated minimization graph
-    // pinned host staging of a minimization's inputs and results, so that
-    // enqueueing it never waits on the device (batched minimization)
-    unsigned char* cg_pinned = nullptr;
-    size_t cg_pinned_bytes = 0;
-    // pinned landing area for the per-call results the host reads back
-    // (energies, force status), so their copies are asynchronous
+    // pinned area for the per-call results the host reads back and a
+    // minimization's state, so their copies are asynchronous
     struct SmallPinned {
         double energy[MEDYAN_FF_COUNT + 1];
         double cg_energy[2 * (MEDYAN_FF_COUNT + 1)];
+        mb::CGState cg_state;
+        mb::LambdaSet cg_lam;
         int force_status;
         int cg_words[4];
         int nl_totals[3];
@@ -274,13 +272,17 @@ cudaError_t launch_pass(medyan_mech* h, int which);
 cudaError_t coords_to_device(medyan_mech* h, const double* host, double* dev, cudaStream_t s);
 // The same through the handle's pinned staging, where staged(h, host) says
 // so, and the way out by plain copies; both ways out wait for the handle's
-// stream and hand out its force status.
+// stream and hand out its force status (unless status is null).
 bool staged(medyan_mech* h, const double* host);
 cudaError_t staged_in(medyan_mech* h, const double* host, double* dev);
-cudaError_t staged_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
+struct HostCopy {
+    const double* dev;
+    double* host;
+};
+cudaError_t staged_out(medyan_mech* h, const HostCopy* c, int n, bool energies, int* status);
 cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
 // A minimization in two halves (cg.cu): enqueue everything on the handle's
-// stream without waiting, then wait and copy the results out.
+// stream, then wait and copy the results out.
 medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double* coord_in);
 medyan_status cg_collect(medyan_mech* h, double* coord_out, double* force_out, medyan_min_result* out);
 cudaError_t coords_to_host(medyan_mech* h, const double* dev, double* host, cudaStream_t s);

@@ -157,7 +157,7 @@ class ForceFieldManager:
     def minimize(self, coord, params: CGParams):
         """CGMethod::minimize on the device. Returns (status, coord, force, MinResult)."""
         x = f64(coord).copy()
-        f = np.zeros_like(x)
+        f = self._out_like(x)
         r = MinResult()
         st = self.lib.medyan_cg_minimize(self.handle, C.byref(params), _dp(x), _dp(f), C.byref(r))
         if st not in (0, 7):
