@@ -14,22 +14,29 @@
 // rounded without contraction (__dmul_rn/__dadd_rn) so the pair set is the
 // oracle's bit for bit.
 //
-// Passes: midpoints + bin index -> bin counts -> scan -> scatter -> sort each
-// bin by cylinder index (deterministic order) -> per-key neighbor counts
-// (27-bin stencil) -> scan -> write pairs / excluded-volume records, and
-// per-plane boundary terms. One host synchronization reads the totals to size
-// the outputs.
+// Passes: midpoints + bin index and boundary counts -> scan of the bins ->
+// scatter -> each bin's records in cylinder order -> per-key neighbor counts
+// (27-bin stencil) -> scan of both lists' counts -> excluded-volume and boundary
+// records. Eight stream operations and one wait: the records go to the buffers
+// of the last build while they hold them (a rebuild of 40,000 cylinders with
+// scans of three kernels, the boundary list apart and the records after a wait
+// for the totals: 143 us; now 72).
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <vector>
 
+#include "device_math.cuh"
 #include "handle.h"
 
 namespace mb {
 
 namespace {
 
-constexpr int kScanBlock = 1024;
+constexpr int kScanThreads = 256, kScanPer = 8, kScanShift = 11;
+constexpr int kScanTile = 1 << kScanShift;
+static_assert(kScanTile == kScanThreads * kScanPer, "a thread scans kScanPer counts");
+constexpr int kFound = 16;  // neighbors of a key that counting keeps for the writing
 
 struct Grid {
     double bin;
@@ -65,10 +72,51 @@ struct CylDev {
     const double* exclk;
 };
 
-__global__ void k_midpoints(CylDev c, const double* __restrict__ x, Grid G, double* __restrict__ mid,
-                            int* __restrict__ cell, int* __restrict__ bin_count, int* __restrict__ err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+// An exclusive scan: entry i is local[i] plus the counts before its tile.
+struct Scan {
+    const int* local;
+    const int* base;
+    __device__ __forceinline__ int operator[](int i) const { return __ldg(local + i) + __ldg(base + (i >> kScanShift)); }
+};
+
+// A binned cylinder, in bin order.
+struct Item {
+    double m[3];
+    int id, fil, pos, cyl;
+};
+
+// Boundary list of a build: its planes and the counts per plane and cylinder.
+struct BoundaryDev {
+    const double4* planes;
+    int n_planes;
+    float cutoff;
+};
+
+// Boundary NL: number of terms of cylinder i against plane p (0, 1 or 2).
+__device__ __forceinline__ int boundary_terms(const CylDev& c, const double* __restrict__ x, const double4& pl,
+                                              float cutoff, int i) {
+    const double* p1 = x + 3 * (size_t)c.b1[i];
+    const double* p2 = x + 3 * (size_t)c.b2[i];
+    // Cylinder::coordinate = midPointCoordinate(b1, b2, 0.5) (Cylinder.cpp:46)
+    double m[3];
+    for (int d = 0; d < 3; ++d) m[d] = p1[d] * (1.0 - 0.5) + 0.5 * p2[d];
+    double dist = (pl.x * m[0] + pl.y * m[1] + pl.z * m[2] + pl.w) / sqrt(pl.x * pl.x + pl.y * pl.y + pl.z * pl.z);
+    if (!(dist < (double)cutoff)) return 0;
+    return (c.minus_end && c.minus_end[i]) ? 2 : 1;
+}
+
+// Thread t < n: midpoint and bin of cylinder t, and its place among the bin's
+// arrivals. Thread n + p n + i: the count of plane p and cylinder i.
+__global__ void k_midpoints(CylDev c, const double* __restrict__ x, Grid G, BoundaryDev B, double* __restrict__ mid,
+                            int* __restrict__ cell, int* __restrict__ slot, int* __restrict__ bin_count,
+                            int* __restrict__ err, int* __restrict__ count) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= c.n) {
+        const int p = t / c.n - 1;
+        if (p < B.n_planes) count[t] = boundary_terms(c, x, B.planes[p], B.cutoff, t % c.n);
+        return;
+    }
+    const int i = t;
     const double* p1 = x + 3 * (size_t)c.b1[i];
     const double* p2 = x + 3 * (size_t)c.b2[i];
     long long idx = 0, stride = 1;
@@ -87,110 +135,114 @@ __global__ void k_midpoints(CylDev c, const double* __restrict__ x, Grid G, doub
         return;
     }
     cell[i] = (int)idx;
-    atomicAdd(bin_count + idx, 1);
+    slot[i] = atomicAdd(bin_count + idx, 1);
 }
 
-// Three-phase exclusive scan of int counts (in place into out[0..n], out[n] = total).
-__global__ void k_scan_blocks(const int* __restrict__ in, int n, int* __restrict__ out, int* __restrict__ sums) {
-    __shared__ int s[kScanBlock];
-    const int i = blockIdx.x * kScanBlock + threadIdx.x;
-    int v = i < n ? in[i] : 0;
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < kScanBlock; o <<= 1) {
-        int t = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-        __syncthreads();
-        s[threadIdx.x] += t;
-        __syncthreads();
+// Sum of v over the block's threads before this one; total: over all.
+__device__ __forceinline__ int block_before(int v, int* warp_sum, int& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int s = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += u;
     }
-    if (i < n) out[i] = s[threadIdx.x] - v;
-    if (threadIdx.x == kScanBlock - 1) sums[blockIdx.x] = s[threadIdx.x];
-}
-__global__ void k_scan_sums(int* __restrict__ sums, int nb, int* __restrict__ total) {
-    // one block: sequential chunks of kScanBlock
-    __shared__ int s[kScanBlock];
-    __shared__ int carry;
-    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();  // the sums of the call before have been read
+    if (lane == 31) warp_sum[warp] = s;
     __syncthreads();
-    for (int base = 0; base < nb; base += kScanBlock) {
-        const int i = base + threadIdx.x;
-        int v = i < nb ? sums[i] : 0;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < kScanBlock; o <<= 1) {
-            int t = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
-        }
-        if (i < nb) sums[i] = s[threadIdx.x] - v + carry;
-        __syncthreads();
-        if (threadIdx.x == kScanBlock - 1) carry += s[threadIdx.x];
-        __syncthreads();
+    int before = s - v;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) {
+        if (w < warp) before += warp_sum[w];
+        total += warp_sum[w];
     }
-    if (threadIdx.x == 0) *total = carry;
-}
-__global__ void k_scan_add(int* __restrict__ out, int n, const int* __restrict__ sums, const int* __restrict__ total) {
-    const int i = blockIdx.x * kScanBlock + threadIdx.x;
-    if (i < n) out[i] += sums[blockIdx.x];
-    if (i == 0) out[n] = *total;
+    return before;
 }
 
-__global__ void k_scatter(int n, const int* __restrict__ cell, const int* __restrict__ start, int* __restrict__ fillc,
-                          int* __restrict__ items) {
+// Exclusive scan of in[0..n) to entries 0..n, the last one the total, in one
+// kernel: each block scans a tile, the last one to end (ticket) the tiles' sums;
+// readers add the two (Scan). No block waits for another.
+__global__ void __launch_bounds__(kScanThreads) k_scan(const int* __restrict__ in, int n, int* __restrict__ local,
+                                                       int* __restrict__ base, unsigned* __restrict__ ticket) {
+    __shared__ int warp_sum[kScanThreads / 32];
+    __shared__ bool last;
+    const int i0 = blockIdx.x * kScanTile + threadIdx.x * kScanPer;
+    int v[kScanPer], sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) v[k] = 0;
+    if (i0 + kScanPer <= n) {  // tiles begin on 16-byte boundaries
+        const int4 a = *reinterpret_cast<const int4*>(in + i0), b = *reinterpret_cast<const int4*>(in + i0 + 4);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kScanPer; ++k)
+            if (i0 + k < n) v[k] = in[i0 + k];
+    }
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k) {
+        const int u = v[k];
+        v[k] = sum;
+        sum += u;
+    }
+    const int before = block_before(sum, warp_sum, total);
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k)
+        if (i0 + k <= n) local[i0 + k] = before + v[k];
+    if (threadIdx.x == 0) {
+        base[blockIdx.x] = total;
+        last = ticket_add(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    int carry = 0;
+    for (int t0 = 0; t0 < (int)gridDim.x; t0 += kScanThreads) {
+        const int t = t0 + threadIdx.x;
+        const int u = t < (int)gridDim.x ? __ldcg(base + t) : 0;
+        const int b = block_before(u, warp_sum, total);
+        if (t < (int)gridDim.x) base[t] = carry + b;
+        carry += total;
+    }
+}
+
+__global__ void k_scatter(int n, const int* __restrict__ cell, const int* __restrict__ slot, Scan start,
+                          int* __restrict__ order) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || cell[i] < 0) return;
-    int slot = atomicAdd(fillc + cell[i], 1);
-    items[start[cell[i]] + slot] = i;
+    if (i < n && cell[i] >= 0) order[start[cell[i]] + slot[i]] = i;
 }
 
-// Deterministic bin contents: each bin sorted by cylinder index.
-__global__ void k_sort_bins(int nbins, const int* __restrict__ start, int* __restrict__ items) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nbins) return;
-    const int s0 = start[b], s1 = start[b + 1];
+// Deterministic bin contents: the first arrival's thread sorts its bin by
+// cylinder index and writes the bin's records.
+__global__ void k_fill_bins(CylDev c, const int* __restrict__ cell, const int* __restrict__ slot, Scan start,
+                            const double* __restrict__ mid, int* __restrict__ order, Item* __restrict__ items) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n || cell[i] < 0 || slot[i] != 0) return;
+    const int s0 = start[cell[i]], s1 = start[cell[i] + 1];
     for (int a = s0 + 1; a < s1; ++a) {
-        int v = items[a], q = a - 1;
-        while (q >= s0 && items[q] > v) {
-            items[q + 1] = items[q];
+        int v = order[a], q = a - 1;
+        while (q >= s0 && order[q] > v) {
+            order[q + 1] = order[q];
             --q;
         }
-        items[q + 1] = v;
+        order[q + 1] = v;
+    }
+    for (int a = s0; a < s1; ++a) {
+        const int j = order[a];
+        const double* m = mid + 3 * (size_t)j;
+        items[a] = Item{{m[0], m[1], m[2]}, c.id[j], c.fil[j], c.pos[j], j};
     }
 }
 
-// d^2 of the midpoints, rounded as written: ((dx*dx + dy*dy) + dz*dz).
-__device__ __forceinline__ double dist2(const double* __restrict__ mid, int i, int j) {
-    double dx = __dadd_rn(mid[3 * (size_t)j], -mid[3 * (size_t)i]);
-    double dy = __dadd_rn(mid[3 * (size_t)j + 1], -mid[3 * (size_t)i + 1]);
-    double dz = __dadd_rn(mid[3 * (size_t)j + 2], -mid[3 * (size_t)i + 2]);
-    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-}
-
-// mode 0: count pairs per key; mode 1: write pairs (key, neighbor) for the
-// standalone build; mode 2: write excluded-volume records (branch-parent pairs
-// skipped, CylinderExclVolume.cpp:85).
-//
-// One warp per key, a lane per bin of its stencil: the bins hold a tenth of a
-// cylinder on average, so one thread per key spent its time on 27 dependent
-// loads in a row (40,000 cylinders: 48 us each for counting and writing, as
-// few blocks as the keys fill at 256 a block; now 19 and 18 us). A key's pairs
-// stay in bin order, dx outermost, then the bin's order; when writing, keys
-// without a pair end at once.
-template <int MODE>
-__global__ void k_pairs(CylDev c, Grid G, const double* __restrict__ mid, const int* __restrict__ cell,
-                        const int* __restrict__ start, const int* __restrict__ items, double rmaxsq, double rminsq,
-                        int skip_branch, int* __restrict__ count, const int* __restrict__ offset,
-                        int2* __restrict__ pairs, int4* __restrict__ ex_bs, double* __restrict__ ex_krs) {
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (i >= c.n) return;
-    const int ci = cell[i];
-    if (ci < 0) return;
-    int out = 0;
-    if (MODE != 0) {
-        out = offset[i];
-        if (offset[i + 1] == out) return;
-    }
+// Neighbors of key i, found by a warp with a lane per bin of its stencil: the
+// bins hold a tenth of a cylinder on average, so one thread per key spent its
+// time on 27 dependent loads in a row (40,000 cylinders: 48 us; a warp 19). A key's pairs
+// are in bin order, dx outermost, then the bin's order. put(k, j): neighbor
+// number k of the key is j; returns their number. All 32 lanes call.
+template <class Put>
+__device__ __forceinline__ int walk_key(const CylDev& c, const Grid& G, int ci, int i, const Scan& start,
+                                        const Item* __restrict__ items, const double* __restrict__ mid, double rmaxsq,
+                                        double rminsq, int skip_branch, Put put) {
+    const int lane = threadIdx.x & 31;
     const int ix = ci % G.g[0], iy = (ci / G.g[0]) % G.g[1], iz = ci / (G.g[0] * G.g[1]);
     const int jx = ix + lane / 9 - 1, jy = iy + lane / 3 % 3 - 1, jz = iz + lane % 3 - 1;
     int q0 = 0, q1 = 0;
@@ -200,47 +252,128 @@ __global__ void k_pairs(CylDev c, Grid G, const double* __restrict__ mid, const 
         q1 = start[cj + 1];
     }
     const int idi = c.id[i], fi = c.fil[i], pi = c.pos[i];
-    auto is_pair = [&](int j) {
-        if (idi <= c.id[j]) return false;
-        if (fi == c.fil[j]) {
-            const int ds = pi - c.pos[j];
+    const double mx = mid[3 * (size_t)i], my = mid[3 * (size_t)i + 1], mz = mid[3 * (size_t)i + 2];
+    auto is_pair = [&](const Item& o) {
+        if (idi <= o.id) return false;
+        if (fi == o.fil) {
+            const int ds = pi - o.pos;
             if ((ds < 0 ? -ds : ds) <= 2) return false;
         }
-        const double d2 = dist2(mid, i, j);
+        // d^2 of the midpoints, rounded as written: ((dx*dx + dy*dy) + dz*dz)
+        const double dx = __dadd_rn(o.m[0], -mx), dy = __dadd_rn(o.m[1], -my), dz = __dadd_rn(o.m[2], -mz);
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
         if (d2 > rmaxsq || d2 < rminsq) return false;
-        return !(skip_branch && c.branching[j] == i);
+        return !(skip_branch && c.branching[o.cyl] == i);
     };
     int n = 0;
     for (int q = q0; q < q1; ++q) n += is_pair(items[q]) ? 1 : 0;
-    if (MODE == 0) {
-        n = __reduce_add_sync(0xffffffffu, n);
-        if (lane == 0) count[i] = n;
-        return;
-    }
+    if (!__any_sync(0xffffffffu, n)) return 0;
     int before = n;  // pairs of the bins before this lane's
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, before, o);
         if (lane >= o) before += v;
     }
-    out += before - n;
+    const int total = __shfl_sync(0xffffffffu, before, 31);
+    before -= n;
     for (int q = q0; q < q1 && n > 0; ++q) {
-        const int j = items[q];
-        if (!is_pair(j)) continue;
-        if (MODE == 1) pairs[out] = make_int2(i, j);
-        if (MODE == 2) {
-            ex_bs[out] = make_int4(3 * c.b1[i], 3 * c.b2[i], 3 * c.b1[j], 3 * c.b2[j]);
+        if (!is_pair(items[q])) continue;
+        put(before, items[q].cyl);
+        ++before;
+        --n;
+    }
+    return total;
+}
+
+// Counts the pairs of each key, a warp per key, and keeps its first neighbors.
+__global__ void k_count_pairs(CylDev c, Grid G, const double* __restrict__ mid, const int* __restrict__ cell, Scan start,
+                              const Item* __restrict__ items, double rmaxsq, double rminsq, int skip_branch,
+                              int* __restrict__ count, int* __restrict__ found) {
+    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= c.n) return;
+    const int ci = cell[i];
+    int n = 0;
+    if (ci >= 0)
+        n = walk_key(c, G, ci, i, start, items, mid, rmaxsq, rminsq, skip_branch, [&](int k, int j) {
+            if (k < kFound) found[(size_t)i * kFound + k] = j;
+        });
+    if (lane == 0) count[i] = n;
+}
+
+// Where the records of a build go: pairs (key, neighbor) of the standalone
+// build, or excluded-volume records (branch-parent pairs skipped,
+// CylinderExclVolume.cpp:85) and boundary records. room: what the buffers hold;
+// lists that do not fit, or of a build with a midpoint outside the grid, are
+// not written. totals (pinned, may be null): pairs, the error flag, boundary
+// terms.
+struct Records {
+    int2* pairs;
+    int4* ex_bs;
+    double* ex_krs;
+    int* b_bs;
+    double2* b_p;
+    int* b_plane;
+    double4* planes;
+    int room, b_room;
+    double b_k, b_slen;
+    int* totals;
+};
+
+// Writes them: thread t < n the pairs of key t from what counting found (all
+// again by the warp when it found more than it kept), thread n + p n + i the
+// terms of plane p and cylinder i.
+template <bool PAIRS>
+__global__ void __launch_bounds__(256) k_write_records(CylDev c, Grid G, BoundaryDev B, const double* __restrict__ mid,
+                                                       const int* __restrict__ cell, Scan start,
+                                                       const Item* __restrict__ items, double rmaxsq, double rminsq,
+                                                       int skip_branch, Scan off, const int* __restrict__ found,
+                                                       const int* __restrict__ err, Records R) {
+    const int m = c.n * (1 + B.n_planes), t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n_pairs = off[c.n], n_terms = off[m] - n_pairs, bad = *err;
+    if (t == 0 && R.totals) {
+        R.totals[0] = n_pairs;
+        R.totals[1] = bad;
+        R.totals[2] = n_terms;
+    }
+    if (bad || n_pairs > R.room || n_terms > R.b_room) return;
+    const int o = t < m ? off[t] : 0, n = t < m ? off[t + 1] - o : 0;
+    auto put = [&](int i, int at, int j) {
+        if constexpr (PAIRS) {
+            R.pairs[at] = make_int2(i, j);
+        } else {
+            R.ex_bs[at] = make_int4(3 * c.b1[i], 3 * c.b2[i], 3 * c.b1[j], 3 * c.b2[j]);
             double k = c.exclk[i];
             if (c.type[i] != c.type[j]) k = k < c.exclk[j] ? c.exclk[j] : k;
-            ex_krs[out] = k * c.eqlen[i] * c.eqlen[j];
+            R.ex_krs[at] = k * c.eqlen[i] * c.eqlen[j];
         }
-        ++out;
-        --n;
+    };
+    if (t < c.n && n <= kFound)
+        for (int k = 0; k < n; ++k) put(t, o + k, found[(size_t)t * kFound + k]);
+    unsigned many = __ballot_sync(0xffffffffu, t < c.n && n > kFound);
+    for (; many; many &= many - 1u) {
+        const int l = __ffs(many) - 1, i = __shfl_sync(0xffffffffu, t, l), at = __shfl_sync(0xffffffffu, o, l);
+        walk_key(c, G, cell[i], i, start, items, mid, rmaxsq, rminsq, skip_branch,
+                 [&](int k, int j) { put(i, at + k, j); });
+    }
+    if constexpr (!PAIRS) {
+        if (t < B.n_planes) R.planes[t] = B.planes[t];
+        if (t < c.n || n == 0) return;
+        const int p = t / c.n - 1, i = t % c.n;
+        int at = o - n_pairs;
+        if (n == 2) {
+            R.b_bs[at] = 3 * c.b1[i];
+            R.b_p[at] = make_double2(R.b_k, R.b_slen);
+            R.b_plane[at] = p;
+            ++at;
+        }
+        R.b_bs[at] = 3 * c.b2[i];
+        R.b_p[at] = make_double2(R.b_k, R.b_slen);
+        R.b_plane[at] = p;
     }
 }
 
 // Canonical order for the standalone build: each key's neighbors ascending.
-__global__ void k_sort_pairs(int n, const int* __restrict__ offset, int2* __restrict__ pairs) {
+__global__ void k_sort_pairs(int n, Scan offset, int2* __restrict__ pairs) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int s0 = offset[i], s1 = offset[i + 1];
@@ -252,45 +385,6 @@ __global__ void k_sort_pairs(int n, const int* __restrict__ offset, int2* __rest
             --q;
         }
         pairs[q + 1] = v;
-    }
-}
-
-// Boundary NL: number of terms of cylinder i against plane p (0, 1 or 2).
-__device__ __forceinline__ int boundary_terms(const CylDev& c, const double* __restrict__ x, const double4& pl,
-                                              float cutoff, int i) {
-    const double* p1 = x + 3 * (size_t)c.b1[i];
-    const double* p2 = x + 3 * (size_t)c.b2[i];
-    // Cylinder::coordinate = midPointCoordinate(b1, b2, 0.5) (Cylinder.cpp:46)
-    double m[3];
-    for (int d = 0; d < 3; ++d) m[d] = p1[d] * (1.0 - 0.5) + 0.5 * p2[d];
-    double dist = (pl.x * m[0] + pl.y * m[1] + pl.z * m[2] + pl.w) / sqrt(pl.x * pl.x + pl.y * pl.y + pl.z * pl.z);
-    if (!(dist < (double)cutoff)) return 0;
-    return (c.minus_end && c.minus_end[i]) ? 2 : 1;
-}
-__global__ void k_boundary_count(CylDev c, const double* __restrict__ x, const double4* __restrict__ planes,
-                                 int n_planes, float cutoff, int* __restrict__ count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    for (int p = 0; p < n_planes; ++p) count[(size_t)p * c.n + i] = boundary_terms(c, x, planes[p], cutoff, i);
-}
-__global__ void k_boundary_write(CylDev c, const double* __restrict__ x, const double4* __restrict__ planes,
-                                 int n_planes, float cutoff, double k, double slen, const int* __restrict__ offset,
-                                 int* __restrict__ bs, double2* __restrict__ bp, int* __restrict__ bplane) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    for (int p = 0; p < n_planes; ++p) {
-        int t = boundary_terms(c, x, planes[p], cutoff, i);
-        if (!t) continue;
-        int o = offset[(size_t)p * c.n + i];
-        if (t == 2) {
-            bs[o] = 3 * c.b1[i];
-            bp[o] = make_double2(k, slen);
-            bplane[o] = p;
-            ++o;
-        }
-        bs[o] = 3 * c.b2[i];
-        bp[o] = make_double2(k, slen);
-        bplane[o] = p;
     }
 }
 
@@ -342,15 +436,18 @@ struct NLBuilder {
     DevBuf<int> b1, b2, id, fil, pos, type, branching, minus_end;
     DevBuf<double> eqlen, exclk;
     DevBuf<double> mid;
-    DevBuf<int> cell, bin_count, bin_start, bin_fill, items, pair_count, pair_off, scan_sums, totals, err;
-    DevBuf<int> bcount, bcount_new, boff;
+    DevBuf<int> cell, slot, bins, bin_start, bin_base, order, off, off_base, found;
+    DevBuf<Item> items;
+    // pairs per key, then boundary terms per plane and cylinder; the load forces read
+    // the boundary membership of the last build that gave the handle its records
+    DevBuf<int> counts, counts_built;
     DevBuf<int2> pairs;
     DevBuf<double4> planes;
     medyan_nl_params nl{};
     medyan_boundary_params bp{};
     std::vector<double> plane_host;
     bool has_boundary = false;
-    bool boundary_built = false;  // bcount holds the last build's plane membership
+    bool boundary_built = false;  // counts_built holds the last build's plane membership
     int n = 0;
 
     CylDev view() const {
@@ -381,116 +478,90 @@ struct NLBuilder {
         return cudaSuccess;
     }
 
-    // scan of cnt[0..m) into off[0..m] (off[m] = total)
-    cudaError_t scan(const int* cnt, int m, int* off, cudaStream_t s) {
-        const int nb = (m + kScanBlock - 1) / kScanBlock;
-        cudaError_t e = scan_sums.reserve(nb + 1);
-        if (e == cudaSuccess) e = totals.reserve(4);
+    int planes_on() const { return has_boundary && bp.n_planes > 0 ? bp.n_planes : 0; }
+    BoundaryDev boundary(bool on) const { return BoundaryDev{planes.raw(), on ? planes_on() : 0, bp.cutoff}; }
+    Scan starts() const { return Scan{bin_start.raw(), bin_base.raw()}; }
+    Scan offsets() const { return Scan{off.raw(), off_base.raw()}; }
+    long long n_bins() const {
+        const Grid G = make_grid(nl);
+        return (long long)G.g[0] * G.g[1] * G.g[2];
+    }
+    int* error() const { return bins.raw() + n_bins(); }
+
+    cudaError_t scan(const int* cnt, int m, DevBuf<int>& local, DevBuf<int>& base, int* ticket, cudaStream_t s) {
+        const int tiles = m / kScanTile + 1;  // of the m + 1 entries
+        cudaError_t e = local.reserve((size_t)m + 1);
+        if (e == cudaSuccess) e = base.reserve(tiles);
         if (e != cudaSuccess) return e;
-        if (m == 0) return cudaMemsetAsync(off, 0, sizeof(int), s);
-        k_scan_blocks<<<nb, kScanBlock, 0, s>>>(cnt, m, off, scan_sums.raw());
-        k_scan_sums<<<1, kScanBlock, 0, s>>>(scan_sums.raw(), nb, totals.raw());
-        k_scan_add<<<nb, kScanBlock, 0, s>>>(off, m, scan_sums.raw(), totals.raw());
+        k_scan<<<tiles, kScanThreads, 0, s>>>(cnt, m, local.raw(), base.raw(), reinterpret_cast<unsigned*>(ticket));
         return cudaGetLastError();
     }
 
-    // Bins the midpoints and counts pairs per key: pair_off[n] is the total,
-    // err whether a midpoint lies outside the grid. Nothing is waited for.
-    medyan_status enqueue_count(const double* x, int skip_branch, cudaStream_t s) {
+    static int blocks_of(long long threads) { return (int)((threads + 255) / 256); }
+
+    // Bins the midpoints, counts pairs per key and (boundary) terms per plane and
+    // cylinder, and scans the counts. Nothing is waited for.
+    medyan_status enqueue_count(const double* x, int skip_branch, bool with_boundary, cudaStream_t s) {
         const Grid G = make_grid(nl);
-        const long long nbins = (long long)G.g[0] * G.g[1] * G.g[2];
+        const long long nbins = n_bins();
         if (nbins > (1LL << 30)) return MEDYAN_ERR_INVALID_ARG;
-        cudaError_t e = mid.reserve(3 * (size_t)std::max(n, 1));
-        if (e == cudaSuccess) e = cell.reserve(std::max(n, 1));
-        if (e == cudaSuccess) e = items.reserve(std::max(n, 1));
-        if (e == cudaSuccess) e = bin_count.reserve(nbins + 1);
-        if (e == cudaSuccess) e = bin_start.reserve(nbins + 1);
-        if (e == cudaSuccess) e = bin_fill.reserve(nbins + 1);
-        if (e == cudaSuccess) e = pair_count.reserve(n + 1);
-        if (e == cudaSuccess) e = pair_off.reserve(n + 1);
-        if (e == cudaSuccess) e = err.reserve(1);
+        const BoundaryDev B = boundary(with_boundary);
+        const int m = n * (1 + B.n_planes);
+        const size_t n1 = n > 0 ? n : 1;
+        cudaError_t e = mid.reserve(3 * n1);
+        if (e == cudaSuccess) e = cell.reserve(n1);
+        if (e == cudaSuccess) e = slot.reserve(n1);
+        if (e == cudaSuccess) e = order.reserve(n1);
+        if (e == cudaSuccess) e = items.reserve(n1);
+        if (e == cudaSuccess) e = found.reserve(kFound * n1);
+        if (e == cudaSuccess) e = counts.reserve((size_t)m + 1);
+        // the other one too, so that no later build has to allocate
+        if (e == cudaSuccess && with_boundary && !boundary_built) e = counts_built.reserve((size_t)m + 1);
+        if (e == cudaSuccess) e = bins.reserve(nbins + 3);  // then the error flag and the scans' tickets
+        if (e == cudaSuccess) e = cudaMemsetAsync(bins.raw(), 0, sizeof(int) * (nbins + 3), s);
         if (e != cudaSuccess) return cuda_status(e);
-        cudaMemsetAsync(bin_count.raw(), 0, sizeof(int) * (nbins + 1), s);
-        cudaMemsetAsync(bin_fill.raw(), 0, sizeof(int) * (nbins + 1), s);
-        cudaMemsetAsync(err.raw(), 0, sizeof(int), s);
-        const int tb = 256, gb = (n + tb - 1) / tb;
-        if (n > 0) k_midpoints<<<gb, tb, 0, s>>>(view(), x, G, mid.raw(), cell.raw(), bin_count.raw(), err.raw());
-        e = scan(bin_count.raw(), (int)nbins, bin_start.raw(), s);
+        if (n > 0)
+            k_midpoints<<<blocks_of(m), 256, 0, s>>>(view(), x, G, B, mid.raw(), cell.raw(), slot.raw(), bins.raw(),
+                                                     error(), counts.raw());
+        e = scan(bins.raw(), (int)nbins, bin_start, bin_base, error() + 1, s);
         if (e != cudaSuccess) return cuda_status(e);
         if (n > 0) {
-            k_scatter<<<gb, tb, 0, s>>>(n, cell.raw(), bin_start.raw(), bin_fill.raw(), items.raw());
-            k_sort_bins<<<(int)((nbins + tb - 1) / tb), tb, 0, s>>>((int)nbins, bin_start.raw(), items.raw());
+            k_scatter<<<blocks_of(n), 256, 0, s>>>(n, cell.raw(), slot.raw(), starts(), order.raw());
+            k_fill_bins<<<blocks_of(n), 256, 0, s>>>(view(), cell.raw(), slot.raw(), starts(), mid.raw(), order.raw(),
+                                                     items.raw());
             const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
-            k_pairs<0><<<key_blocks(), tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
-                                                   (double)rmaxsq, (double)rminsq, skip_branch, pair_count.raw(), nullptr,
-                                                   nullptr, nullptr, nullptr);
+            k_count_pairs<<<blocks_of(32LL * n), 256, 0, s>>>(view(), G, mid.raw(), cell.raw(), starts(), items.raw(),
+                                                              (double)rmaxsq, (double)rminsq, skip_branch, counts.raw(),
+                                                              found.raw());
         }
-        return cuda_status(scan(pair_count.raw(), n, pair_off.raw(), s));
+        return cuda_status(scan(counts.raw(), m, off, off_base, error() + 2, s));
     }
 
-    int key_blocks() const { return (int)((32LL * n + 255) / 256); }  // a warp per key
+    template <bool PAIRS>
+    cudaError_t enqueue_write(int skip_branch, const Records& R, cudaStream_t s) {
+        const BoundaryDev B = boundary(!PAIRS);
+        const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
+        const long long threads = (long long)n * (1 + B.n_planes);  // at least one block copies the planes
+        k_write_records<PAIRS><<<blocks_of(threads > B.n_planes ? threads : B.n_planes + 1), 256, 0, s>>>(
+            view(), make_grid(nl), B, mid.raw(), cell.raw(), starts(), items.raw(), (double)rmaxsq, (double)rminsq,
+            skip_branch, offsets(), found.raw(), error(), R);
+        return cudaGetLastError();
+    }
 
-    // The same, waited for; returns the pair total.
+    // The count, waited for; returns the pair total.
     medyan_status count_pairs(const double* x, int skip_branch, cudaStream_t s, long long* total) {
-        const medyan_status st = enqueue_count(x, skip_branch, s);
+        const medyan_status st = enqueue_count(x, skip_branch, false, s);
         if (st != MEDYAN_OK) return st;
-        cudaError_t e = cudaSuccess;
-        int h[2] = {0, 0};
-        e = cudaMemcpyAsync(&h[0], pair_off.raw() + n, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h[1], err.raw(), sizeof(int), cudaMemcpyDeviceToHost, s);
+        int h[3] = {0, 0, 0};
+        cudaError_t e = cudaMemcpyAsync(&h[0], off.raw() + n, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(&h[1], off_base.raw() + (n >> kScanShift), sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h[2], error(), sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e);
-        if (h[1]) return MEDYAN_ERR_OUT_OF_GRID;
-        *total = h[0];
+        if (h[2]) return MEDYAN_ERR_OUT_OF_GRID;
+        *total = h[0] + h[1];
         return MEDYAN_OK;
-    }
-
-    template <int MODE>
-    void write_pairs(const double* x, int skip_branch, int2* out_pairs, int4* ex_bs, double* ex_krs, cudaStream_t s) {
-        (void)x;
-        const Grid G = make_grid(nl);
-        const int tb = 256, gb = (n + tb - 1) / tb;
-        if (n == 0) return;
-        const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
-        k_pairs<MODE><<<key_blocks(), tb, 0, s>>>(view(), G, mid.raw(), cell.raw(), bin_start.raw(), items.raw(),
-                                        (double)rmaxsq, (double)rminsq, skip_branch, nullptr, pair_off.raw(),
-                                        out_pairs, ex_bs, ex_krs);
-        if (MODE == 1) k_sort_pairs<<<gb, tb, 0, s>>>(n, pair_off.raw(), out_pairs);
-    }
-
-    // Boundary NL, in two halves: counts per plane and cylinder into bcount_new
-    // (boff[n_planes n] is the total), then the handle's boundary records. The
-    // plane membership that the load forces read (bcount) changes with the
-    // second half only.
-    bool boundary_on() const { return has_boundary && bp.n_planes > 0; }
-    medyan_status enqueue_boundary_count(const double* x, cudaStream_t s) {
-        const int np = bp.n_planes;
-        cudaError_t e = bcount_new.reserve((size_t)np * n + 1);
-        if (e == cudaSuccess) e = boff.reserve((size_t)np * n + 1);
-        if (e != cudaSuccess) return cuda_status(e);
-        const int tb = 256, gb = (n + tb - 1) / tb;
-        if (n > 0) k_boundary_count<<<gb, tb, 0, s>>>(view(), x, planes.raw(), np, bp.cutoff, bcount_new.raw());
-        return cuda_status(scan(bcount_new.raw(), np * n, boff.raw(), s));
-    }
-    medyan_status write_boundary(medyan_mech* h, const double* x, int tot, cudaStream_t s) {
-        const int np = bp.n_planes, tb = 256, gb = (n + tb - 1) / tb;
-        cudaError_t e = h->boundary_bs.reserve(tot);
-        if (e == cudaSuccess) e = h->boundary_p.reserve(tot);
-        if (e == cudaSuccess) e = h->boundary_plane.reserve(tot);
-        if (e == cudaSuccess) e = h->planes.reserve(np);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(h->planes.raw(), planes.raw(), sizeof(double4) * np, cudaMemcpyDeviceToDevice, s);
-        if (e != cudaSuccess) return cuda_status(e);
-        if (n > 0 && tot > 0)
-            k_boundary_write<<<gb, tb, 0, s>>>(view(), x, planes.raw(), np, bp.cutoff, bp.k, bp.screen_length,
-                                               boff.raw(), h->boundary_bs.raw(), h->boundary_p.raw(),
-                                               h->boundary_plane.raw());
-        h->ff.n_boundary = tot;
-        h->ff.n_planes = np;
-        bcount.swap(bcount_new);
-        e = cudaGetLastError();
-        boundary_built = e == cudaSuccess;
-        return cuda_status(e);
     }
 
     std::vector<double4> planes_host4() const {
@@ -542,8 +613,15 @@ medyan_status medyan_nl_build(const medyan_cylinders* cyl, const double* coord, 
                 else if (total > 0) {
                     e = b.pairs.reserve(total);
                     if (e == cudaSuccess) {
-                        b.write_pairs<1>(x.raw(), 0, b.pairs.raw(), nullptr, nullptr, s);
-                        e = cudaMemcpyAsync(pairs_out, b.pairs.raw(), sizeof(int2) * total, cudaMemcpyDeviceToHost, s);
+                        Records R{};
+                        R.pairs = b.pairs.raw();
+                        R.room = (int)total;
+                        e = b.enqueue_write<true>(0, R, s);
+                        if (e == cudaSuccess) {
+                            k_sort_pairs<<<NLBuilder::blocks_of(b.n), 256, 0, s>>>(b.n, b.offsets(), b.pairs.raw());
+                            e = cudaGetLastError();
+                        }
+                        if (e == cudaSuccess) e = cudaMemcpyAsync(pairs_out, b.pairs.raw(), sizeof(int2) * total, cudaMemcpyDeviceToHost, s);
                     }
                     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
                     if (e != cudaSuccess) st = cuda_status(e);
@@ -599,28 +677,56 @@ medyan_status medyan_mech_rebuild_neighbors(medyan_mech* h, int64_t* n_excl_out,
     if (!h || !h->nl) return MEDYAN_ERR_INVALID_ARG;
     NLBuilder* b = reinterpret_cast<NLBuilder*>(h->nl);
     cudaStream_t s = h->stream;
-    // both lists' counts, then one wait for their totals
+    bool written = false;
+    // both lists' counts and, where the handle's buffers have room, the records; one
+    // wait for the totals. The records come again when they did not fit.
     int* tot = h->small->nl_totals;  // pairs, outside the grid, boundary terms
     tot[0] = tot[1] = tot[2] = 0;
-    medyan_status st = b->enqueue_count(h->x.raw(), 1, s);
-    if (st == MEDYAN_OK && b->boundary_on()) st = b->enqueue_boundary_count(h->x.raw(), s);
+    medyan_status st = b->enqueue_count(h->x.raw(), 1, true, s);
     if (st != MEDYAN_OK) return st;
-    cudaError_t e = cudaMemcpyAsync(tot, b->pair_off.raw() + b->n, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(tot + 1, b->err.raw(), sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess && b->boundary_on())
-        e = cudaMemcpyAsync(tot + 2, b->boff.raw() + (size_t)b->bp.n_planes * b->n, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    const int np = b->planes_on();
+    auto write = [&] {
+        Records R{};
+        R.ex_bs = h->excl_bs.raw();
+        R.ex_krs = h->excl_krs.raw();
+        R.room = (int)std::min({h->excl_bs.cap, h->excl_krs.cap, (size_t)INT_MAX});
+        R.b_bs = h->boundary_bs.raw();
+        R.b_p = h->boundary_p.raw();
+        R.b_plane = h->boundary_plane.raw();
+        R.planes = h->planes.raw();
+        R.b_room = (int)std::min({h->boundary_bs.cap, h->boundary_p.cap, h->boundary_plane.cap, (size_t)INT_MAX});
+        if (h->planes.cap < (size_t)np) R.b_room = -1;
+        R.b_k = b->bp.k;
+        R.b_slen = b->bp.screen_length;
+        R.totals = tot;
+        cudaError_t e = b->enqueue_write<false>(1, R, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        written = e == cudaSuccess && !tot[1] && tot[0] <= R.room && tot[2] <= R.b_room;
+        return e;
+    };
+    cudaError_t e = write();
     if (e != cudaSuccess) return cuda_status(e);
     if (tot[1]) return MEDYAN_ERR_OUT_OF_GRID;
-    e = h->excl_bs.reserve(tot[0]);
-    if (e == cudaSuccess) e = h->excl_krs.reserve(tot[0]);
+    // a list that outgrows its buffer gets an eighth more: moving beads change it a little each time
+    auto fit = [](auto& buf, size_t count) {
+        cudaError_t e = count <= buf.cap && buf.raw() ? cudaSuccess : buf.reserve(buf.cap > 1 ? count + count / 8 : count);
+        return e == cudaSuccess ? buf.reserve(count) : e;
+    };
+    e = fit(h->excl_bs, tot[0]);
+    if (e == cudaSuccess) e = fit(h->excl_krs, tot[0]);
+    if (e == cudaSuccess && np > 0) e = fit(h->boundary_bs, tot[2]);
+    if (e == cudaSuccess && np > 0) e = fit(h->boundary_p, tot[2]);
+    if (e == cudaSuccess && np > 0) e = fit(h->boundary_plane, tot[2]);
+    if (e == cudaSuccess && np > 0) e = h->planes.reserve(np);
+    if (e == cudaSuccess && !written) e = write();
     if (e != cudaSuccess) return cuda_status(e);
-    b->write_pairs<2>(h->x.raw(), 1, nullptr, h->excl_bs.raw(), h->excl_krs.raw(), s);
     h->ff.n_excl = tot[0];
     const int nb = tot[2];
-    if (b->boundary_on()) {
-        st = b->write_boundary(h, h->x.raw(), nb, s);
-        if (st != MEDYAN_OK) return st;
+    if (np > 0) {
+        h->ff.n_boundary = nb;
+        h->ff.n_planes = np;
+        b->counts.swap(b->counts_built);
+        b->boundary_built = true;
     }
     st = refresh_device_ff(h);
     if (st != MEDYAN_OK) return st;
@@ -699,7 +805,7 @@ extern "C" medyan_status medyan_mech_boundary_load_forces(medyan_mech* h, const 
     if (e == cudaSuccess) e = out.reserve(tot);
     if (e != cudaSuccess) return cuda_status(e);
     const int g = nt < 148 * 8 ? nt : 148 * 8;
-    k_boundary_load<<<g, 128, 0, s>>>(b->view(), h->x.raw(), b->planes.raw(), b->bp.n_planes, b->bcount.raw(),
+    k_boundary_load<<<g, 128, 0, s>>>(b->view(), h->x.raw(), b->planes.raw(), b->bp.n_planes, b->counts_built.raw() + b->n,
                                       b->bp.k, b->bp.screen_length, nt, cyl.raw(), plus.raw(), nmon.raw(),
                                       mon.raw(), doff.raw(), out.raw());
     e = cudaGetLastError();
