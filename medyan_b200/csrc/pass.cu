@@ -845,7 +845,14 @@ int g_num_sms = 148;  // SMs of the device (set at init; B200: 148)
 PassGeometry pass_geometry(const ChainDev& ch, const DeviceFF& ff, bool stream) {
     PassGeometry g{};
     g.threads = kPassThreads;
-    g.excl_threads = excl_block_of(ff) > 128 ? 128 : excl_block_of(ff);
+    // Without a size of the caller's, a pair per thread takes the largest block:
+    // half the rows and tickets of 64-thread blocks (evaluate pass of the
+    // 400k-cylinder network 33.4 -> 32.8 us mixed, 35.3 -> 34.5 FP64, 100k cylinders
+    // 22.3 -> 21.1). Four lanes per pair, in small networks, keep 64, which
+    // spreads their few pairs over twice the SMs.
+    g.excl_quad = ff.n_excl <= kQuadPairs;
+    g.excl_threads = ff.excl_block <= 0 && !g.excl_quad ? kExclThreadsMax
+                     : excl_block_of(ff) > kExclThreadsMax ? kExclThreadsMax : excl_block_of(ff);
     const int tiles = (ch.n_pos + kWarpOut - 1) / kWarpOut;
     const int warps = g.threads / 32;
     g.nch = (tiles + warps - 1) / warps;
@@ -860,7 +867,6 @@ PassGeometry pass_geometry(const ChainDev& ch, const DeviceFF& ff, bool stream) 
     const int cap = g_num_sms * kMainBlocksPerSM;
     g.main_blocks = units < 1 ? 1 : (units < cap ? units : cap);
     g.branch_blocks = (ff.n_branch + g.threads - 1) / g.threads;
-    g.excl_quad = ff.n_excl <= kQuadPairs;
     const int per = g.excl_quad ? g.excl_threads / 4 : g.excl_threads;
     const int eb = (ff.n_excl + per - 1) / per;
     const int ecap = g_num_sms * 32;
