@@ -252,6 +252,11 @@ __device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double
     const Sink<FIXED> t{status};
     bool bad = false;
     int f_blocks = 0;  // blocks that the force tasks fill
+    // The pairs' forces, the longest tasks, take four warps of a block, one per
+    // scheduler, where a quarter of the team holds them so: two of their FP64
+    // chains on one scheduler wait for each other (11,700 cycles of a pass against
+    // 10,500 at 50 filaments of 10 cylinders).
+    const bool spread = ((ff.n_excl + 7) / 8 + 3) / 4 * 4 <= tm.size;
     if (force) {
         // lane l: tasks of kind l, and the end of their numbers
         const int n = lane == FX ? ff.n_excl : lane == FB ? ff.n_branch : lane == FC ? a.ch.n_pos : lane == FLinker ? ff.n_linker
@@ -259,6 +264,7 @@ __device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double
                     : lane == FBend ? ff.n_bend : 0;
         const int per = lane == FX ? 8 : lane == FC ? kWarpOut : 32;
         int end = (n + per - 1) / per;
+        if (spread && lane == FX) end = (end + 3) / 4 * kWarps;
 #pragma unroll
         for (int o = 1; o < kFKinds; o <<= 1) {
             const int v = __shfl_up_sync(kFull, end, o);
@@ -271,9 +277,13 @@ __device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double
         for (int task = tm.rank * kWarps + warp; task < total; task += tm.size * kWarps) {
             const int kind = __popc(__ballot_sync(kFull, end <= task) & ((1u << kFKinds) - 1u));
             const int before = __shfl_sync(kFull, end, kind > 0 ? kind - 1 : 0);
-            const int i = kind > 0 ? task - before : task;
+            int i = kind > 0 ? task - before : task;
             double none[4];
             if (kind == FX) {
+                if (spread) {
+                    if (warp >= 4) continue;
+                    i = i / kWarps * 4 + warp;
+                }
                 const int p = i * 8 + (lane >> 2), pc = min(p, ff.n_excl - 1);
                 const int4 q = __ldg(ff.excl_bs + pc);
                 const double krs = __ldg(ff.excl_krs + pc);
@@ -300,10 +310,21 @@ __device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double
     if (K > 0) {
         int rounds = sm.n_rows * K, alt = 0;
         const int group = threadIdx.x / kVecThreads, gthread = threadIdx.x % kVecThreads, gwarp = warp & 7;
-        int first = (tm.rank - f_blocks) % tm.size;
-        if (first < 0) first += tm.size;
+        // Up to two rounds a block fit beside the forces, on the blocks without
+        // tasks; more go round the whole team. Rounds that come round to the first
+        // blocks, which have the pairs, end the pass (12,000 cycles there, 9,600 without;
+        // with the spread of the pairs a minimization of 500 x 20 cylinders
+        // takes 17.6 ms, before 18.5, of 900 x 13 2.73 and 3.02, of 130 x 15 21.9 and 23.1).
+        int first = tm.rank - f_blocks, width = tm.size;
+        if (f_blocks < tm.size && rounds <= 2 * kVecGroups * (tm.size - f_blocks)) {
+            width -= f_blocks;
+            if (first < 0) first = rounds;  // none here
+        } else {
+            first %= tm.size;
+            if (first < 0) first += tm.size;
+        }
 #pragma unroll 1
-        for (int round = first * kVecGroups + group; round < rounds; round += tm.size * kVecGroups, alt ^= 1) {
+        for (int round = first * kVecGroups + group; round < rounds; round += width * kVecGroups, alt ^= 1) {
             int kind = 0, v = round, k = 0;
             while (v >= sm.rows[kind] * K) v -= sm.rows[kind++] * K;
             while (v >= sm.rows[kind]) {

@@ -103,3 +103,24 @@ def test_forces_after_failed_line_searches(gpu_lib):
             assert s == 0 and np.array_equal(fg, ff.compute_forces(xg)), (limit, counts(r))
             failed += r.num_force_call < r.num_iter
         assert failed > 0  # some runs ended after a failed line search
+
+
+@pytest.mark.parametrize("size", [(7, 6, 800.0), (83, 10, 1600.0), (500, 20, 3200.0), (2400, 20, 5500.0)])
+def test_energies_are_the_energy_kernels(gpu_lib, size):
+    """The loop's energies are the per-potential kernels' bit for bit, from a few
+    energy rows to shares of more than 32 rows (the largest size), and on teams
+    where the rounds have blocks of their own and where they do not."""
+    n_fil, n_cyl, box = size
+    net = make_workload(0, n_fil=n_fil, cyl_per_fil=n_cyl, box=box, n_linker=n_fil, n_branch=n_fil // 4,
+                        n_motor=n_fil // 8, seed=11)
+    with ForceFieldManager("fp64") as ff:
+        ff.vectorize_all_force_fields(net.system_view())
+        ff.set_coords(net.flat_coords())
+        ff.set_cylinders(net.cylinders_view(), net.nl_params(), net.boundary_params()[0])
+        ff.rebuild_neighbor_lists()
+        s, x, f, r = ff.minimize(net.flat_coords(), cgp(energy_call_limit=30))
+        ff.set_shapes(pass_layout=1)
+        before = ff.compute_individual_energies(net.flat_coords()).as_array()
+        after = ff.compute_individual_energies(x).as_array()
+    assert s == 0
+    assert np.array_equal(before, np.array(r.energy_before)) and np.array_equal(after, np.array(r.energy_after))
