@@ -869,6 +869,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
     Smem& sm = smem();
+    cluster.sync();  // a block's shared memory may be written once the block is known to have started
     for (;;) {
         __syncthreads();
         if (cluster.block_rank() == 0 && threadIdx.x == 0) {
