@@ -702,6 +702,7 @@ static LoopArgs loop_args(medyan_mech* h, const CGLaunch& c) {
     a.st = c.st;
     a.lam = c.L;
     a.eout = h->cg_eout.raw();
+    a.e_last = h->energy_out.raw();
     a.erow = h->cg_rows.raw();
     a.vrow = h->cg_rows.raw() + loop_erow_doubles(loop_row_count(h->chain, h->ff));
     a.words = h->cg_words.raw();

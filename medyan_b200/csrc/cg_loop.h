@@ -19,6 +19,7 @@ struct LoopArgs {
     CGState* st;       // parameters in, final state out
     LambdaSet* lam;    // pending step sizes when the loop hands over
     double* eout;      // [2][MEDYAN_FF_COUNT + 1]: energies before and after
+    double* e_last;    // MEDYAN_FF_COUNT + 1: as an energy pass at the final coordinates leaves them; may be null
     double* erow;      // [2][kMaxLambda][4][loop_row_count]
     double* vrow;      // [2][vb, or the 8 warps of a single one][4]: of the sums, of max|d|
     int* words;        // kLoopWords words, zero at the launch

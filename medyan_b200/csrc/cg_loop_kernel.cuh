@@ -840,11 +840,15 @@ __device__ void minimize() {
         sm.L.lam[0] = 0.0;
     }
     if (!team_sync()) return leave(kLoopLost);
-    if (s.status != MEDYAN_ERR_LINE_SEARCH) {
+    // after a failed line search they are not part of the result, but a single
+    // network's energy buffer holds those of its coordinates all the same
+    const bool failed = s.status == MEDYAN_ERR_LINE_SEARCH;
+    if (!failed || a.e_last) {
         pass<R, FIXED>(at_x, 1, false, 0.0, nullptr, nullptr, parity);
         if (!team_sync()) return leave(kLoopLost);
         if (!add_rows<BATCH>(1, parity)) return leave(kLoopHandOver);
-        record(1);
+        if (a.e_last && tm.rank == 0 && threadIdx.x < kOut) a.e_last[threadIdx.x] = sm.out[threadIdx.x];
+        if (!failed) record(1);
         __syncthreads();
     }
     leave(kLoopDone);
