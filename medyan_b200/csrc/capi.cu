@@ -2,6 +2,9 @@
 // host-side validation and packing of the vectorized force fields, and the
 // energy/force entry points. The minimizer and the neighbor list are in
 // cg.cu and nl.cu.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -363,8 +366,8 @@ cudaError_t coords_to_host(medyan_mech* h, const double* dev, double* host, cuda
 // operation of its own: an evaluation was four copies, a memset and two waits
 // around a pass of 10 us. Pinned memory takes over 1 ms to allocate from about
 // 2 MB on, so the staging is four pieces whatever the network's size. Evaluations
-// before and now: 550 beads 67 and 40 us, 10,500 142 and 76, 42,000 337 and
-// 212, 420,000 2,265 and 1,850.
+// by plain copies and now: 550 beads 61 and 40 us, 5,400 81 and 53, 10,500 91 and 69,
+// 21,000 117 and 107; larger networks copy plainly (kStageBoth).
 constexpr int kIoThreads = 256;
 constexpr int kIoBeads = 5460;  // beads a piece: 128 KB
 
@@ -396,14 +399,8 @@ __global__ void k_hand_out(int n3, int i0, const int* __restrict__ pos, const do
     }
 }
 
-// Whether a copy to or from host goes through the staging, which the first such
-// call makes. Memory that CUDA knows (pinned, managed) takes plain copies, which
-// need no host time there, as does everything when no staging is to be had.
-bool staged(medyan_mech* h, const double* host) {
-    cudaPointerAttributes a;
-    if (h->n_beads == 0 || cudaSetDevice(h->device) != cudaSuccess ||
-        cudaPointerGetAttributes(&a, host) != cudaSuccess || a.type != cudaMemoryTypeUnregistered)
-        return false;
+// The staging, made once; false when there is none to be had.
+static bool make_staging(medyan_mech* h) {
     if (h->io) return true;
     const int slots = h->n_beads > kIoBeads ? kIoSlots : 2;  // two arrays go out together
     const int beads = h->n_beads < kIoBeads ? h->n_beads : kIoBeads;
@@ -417,6 +414,17 @@ bool staged(medyan_mech* h, const double* host) {
         cudaGetLastError();
     }
     return e == cudaSuccess;
+}
+
+// Whether a copy to or from host goes through the staging: up to the size that
+// the call says (a kStage constant, handle.h). Memory that CUDA knows (pinned,
+// managed) takes plain copies, which need no host time there, as does everything
+// when no staging is to be had.
+bool staged(medyan_mech* h, const double* host, int most) {
+    if (most == kStageIn && h->n_beads < kStageInLeast && h->identity_order) return false;
+    cudaPointerAttributes a;
+    return h->n_beads > 0 && h->n_beads <= most && cudaSetDevice(h->device) == cudaSuccess &&
+           cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeUnregistered && make_staging(h);
 }
 
 // Piece k in slot s: its first bead and number of beads, in the caller's order.
@@ -476,10 +484,26 @@ cudaError_t staged_out(medyan_mech* h, const HostCopy* c, int n, bool energies, 
     return e;
 }
 
+// Brings the whole pages of an output into memory, while the device works: the
+// driver's plain copy takes a fault for each page that was never touched (forces
+// of 420,000 beads into new memory 4.9 ms, so 3.1; through the staging 3.3; into memory
+// in use 0.55). The contents stay. Without the advice the faults stay too.
+void populate_output(const medyan_mech* h, const double* host) {
+#ifdef MADV_POPULATE_WRITE
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, host) != cudaSuccess || at.type != cudaMemoryTypeUnregistered) return;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE),
+                    a = (reinterpret_cast<uintptr_t>(host) + page - 1) / page * page,
+                    b = reinterpret_cast<uintptr_t>(host + 3 * (size_t)h->n_beads) / page * page;
+    if (a < b) madvise(reinterpret_cast<void*>(a), b - a, MADV_POPULATE_WRITE);
+#endif
+}
+
 // The same by plain copies.
 cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status) {
     cudaStream_t s = h->stream;
     cudaError_t e = cudaSuccess;
+    populate_output(h, host);
     if (energies)
         e = cudaMemcpyAsync(h->small->energy, h->energy_out.ptr(), sizeof h->small->energy, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = coords_to_host(h, dev, host, s);
@@ -714,7 +738,10 @@ medyan_status medyan_mech_destroy(medyan_mech* h) {
 
 medyan_status medyan_mech_set_coords(medyan_mech* h, const double* coord) {
     if (!h || (!coord && h->n_beads)) return MEDYAN_ERR_INVALID_ARG;
-    cudaError_t e = staged(h, coord) ? staged_in(h, coord, h->x.raw()) : coords_to_device(h, coord, h->x.raw(), h->stream);
+    // what follows this call uses it: not in the first evaluation's time
+    if (h->n_beads > 0 && h->n_beads <= kStageMinimize && cudaSetDevice(h->device) == cudaSuccess) make_staging(h);
+    cudaError_t e = staged(h, coord, kStageIn) ? staged_in(h, coord, h->x.raw())
+                                               : coords_to_device(h, coord, h->x.raw(), h->stream);
     if (e != cudaSuccess) return cuda_status(e);
     return sync_status(h);
 }
@@ -747,7 +774,7 @@ medyan_status medyan_mech_forces(medyan_mech* h, double* force_out) {
     if (e != cudaSuccess) return cuda_status(e);
     int status = 0;
     const HostCopy to{h->f.raw(), force_out};
-    if (staged(h, force_out)) e = staged_out(h, &to, 1, false, &status);
+    if (staged(h, force_out, kStageOut)) e = staged_out(h, &to, 1, false, &status);
     else e = plain_out(h, h->f.raw(), force_out, false, &status);
     if (e != cudaSuccess) return cuda_status(e);
     return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
@@ -811,7 +838,7 @@ medyan_status medyan_mech_device_buffers(medyan_mech* h, double** coord, double*
 medyan_status medyan_mech_evaluate(medyan_mech* h, const double* coord, double* e_total, double* e_per_ff,
                                    double* force_out) {
     if (!h || !coord || !e_total || !force_out) return MEDYAN_ERR_INVALID_ARG;
-    const bool in = staged(h, coord);
+    const bool in = staged(h, coord, kStageBoth);
     cudaError_t e = in ? staged_in(h, coord, h->x.raw()) : coords_to_device(h, coord, h->x.raw(), h->stream);
     if (e != cudaSuccess) return cuda_status(e);
     e = launch_pass(h, kPassBoth);
@@ -821,8 +848,8 @@ medyan_status medyan_mech_evaluate(medyan_mech* h, const double* coord, double* 
     }
     int status = 0;
     const HostCopy to{h->f.raw(), force_out};
-    e = staged(h, force_out) ? staged_out(h, &to, 1, true, &status)
-                             : plain_out(h, h->f.raw(), force_out, true, &status);
+    e = staged(h, force_out, kStageBoth) ? staged_out(h, &to, 1, true, &status)
+                                         : plain_out(h, h->f.raw(), force_out, true, &status);
     if (e != cudaSuccess) return cuda_status(e);
     const double* out = h->small->energy;
     *e_total = out[MEDYAN_FF_COUNT];

@@ -735,7 +735,7 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     if (e == cudaSuccess && h->cg_team > 0) e = init_cg_loop();
     if (e != cudaSuccess) return cuda_status(e);
     const CGLaunch c = make_launch(h);
-    e = staged(h, coord_in) ? staged_in(h, coord_in, c.x) : coords_to_device(h, coord_in, c.x, s);
+    e = staged(h, coord_in, kStageMinimize) ? staged_in(h, coord_in, c.x) : coords_to_device(h, coord_in, c.x, s);
     if (e == cudaSuccess) e = cg_start(h, c, s);
     if (e == cudaSuccess && h->cg_team > 0) {
         e = cudaMemsetAsync(h->cg_words.raw(), 0, sizeof(int) * kLoopWords, s);
@@ -773,10 +773,11 @@ medyan_status cg_collect(medyan_mech* h, double* coord_out, double* force_out, m
     const HostCopy to[2] = {{h->x.raw(), coord_out}, {h->f.raw(), force_out}};
     const int n = force_out ? 2 : 1;
     bool by_stage = true;
-    for (int i = 0; i < n; ++i) by_stage = by_stage && staged(h, to[i].host);
+    for (int i = 0; i < n; ++i) by_stage = by_stage && staged(h, to[i].host, kStageMinimize);
     if (by_stage) {
         if (e == cudaSuccess) e = staged_out(h, to, n, false, nullptr);
     } else {
+        if (force_out) populate_output(h, force_out);
         for (int i = 0; i < n && e == cudaSuccess; ++i) e = coords_to_host(h, to[i].dev, to[i].host, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }

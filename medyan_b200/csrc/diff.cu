@@ -346,11 +346,12 @@ int blocks_for(int n) {
 }
 
 // Uploads v (caller's order) into h->hv_v (internal order).
-cudaError_t upload_direction(medyan_mech* h, const double* v) {
+// most: what the call stages (kStageIn, or kStageBoth with a result of the same size)
+cudaError_t upload_direction(medyan_mech* h, const double* v, int most) {
     const int n3 = 3 * h->n_beads;
     cudaError_t e = h->hv_v.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess)
-        e = staged(h, v) ? staged_in(h, v, h->hv_v.raw()) : coords_to_device(h, v, h->hv_v.raw(), h->stream);
+        e = staged(h, v, most) ? staged_in(h, v, h->hv_v.raw()) : coords_to_device(h, v, h->hv_v.raw(), h->stream);
     return e;
 }
 
@@ -384,7 +385,7 @@ extern "C" medyan_status medyan_mech_param_grad(medyan_mech* h, int32_t ff, cons
     DevBuf<double>& gp = h->pg_p;
     cudaError_t ce = gk.reserve(count);
     if (ce == cudaSuccess) ce = gp.reserve(count);
-    if (ce == cudaSuccess && v) ce = upload_direction(h, v);
+    if (ce == cudaSuccess && v) ce = upload_direction(h, v, kStageIn);
     if (ce != cudaSuccess) return cuda_status(ce);
     const double* dv = v ? h->hv_v.raw() : nullptr;
     const int g = (count + kThreads - 1) / kThreads;
@@ -416,7 +417,7 @@ extern "C" medyan_status medyan_mech_hvp(medyan_mech* h, const double* v, double
     if (n3 == 0) return MEDYAN_OK;
     cudaStream_t s = h->stream;
     cudaError_t ce = h->hv_a.reserve(n3);
-    if (ce == cudaSuccess) ce = upload_direction(h, v);
+    if (ce == cudaSuccess) ce = upload_direction(h, v, kStageBoth);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(h->hv_a.raw(), 0, sizeof(double) * n3, s);
     if (ce != cudaSuccess) return cuda_status(ce);
     const double* x = h->x.raw();
@@ -447,7 +448,8 @@ extern "C" medyan_status medyan_mech_hvp(medyan_mech* h, const double* v, double
     int status = 0;
     const HostCopy to{out, hv};
     if (ce == cudaSuccess)
-        ce = staged(h, hv) ? staged_out(h, &to, 1, false, &status) : plain_out(h, out, hv, false, &status);
+        ce = staged(h, hv, kStageBoth) ? staged_out(h, &to, 1, false, &status)
+                                       : plain_out(h, out, hv, false, &status);
     if (ce != cudaSuccess) return cuda_status(ce);
     return status ? MEDYAN_ERR_NONFINITE : MEDYAN_OK;
 }

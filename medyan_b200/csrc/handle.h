@@ -19,6 +19,21 @@ namespace mb {
 
 struct medyan_async;  // async.cu
 constexpr int kIoSlots = 4;  // pieces of the staging of host coordinates
+// Largest networks (beads) whose host arrays go through the staging, by what the
+// call moves; larger ones take plain copies. Two things meet here: the staging
+// saves the copies' fixed cost, but one host thread fills it at 12 GB/s, where
+// the driver copies pageable memory at 20. Staged and plain, us, results in memory
+// that is in use:
+//   coordinates in: 85 beads 16.7 and 13.8 (in chain order, else 16.3 and 19.3), 550
+//     17.4 and 19.2, 2,700 beads 21.6 and 47.4, 5,400 25.4 and 22.5, 42,000 90 and
+//     71, 420,000 900 and 514 (the driver's copies up to 64 KB take another way)
+//   forces out: 30,000 82 and 90, 42,000 105 and 107, 60,000 154 and 133
+//   both (evaluate): 21,000 105 and 120, 27,000 134 and 135, 33,000 163 and 156,
+//     60,000 277 and 235, 420,000 1,822 and 1,070 (Hessian-vector products alike)
+//   minimization, 8 energy calls: 60,000 675 and 737, 84,000 712 and 641, 126,000
+//     1,000 and 849, 420,000 3,061 and 2,263
+constexpr int kStageIn = 2730, kStageOut = 42000, kStageBoth = 30000, kStageMinimize = 72000;
+constexpr int kStageInLeast = 350;  // coordinates in, in chain order
 
 template <class T>
 struct DevBuf {
@@ -270,16 +285,19 @@ cudaError_t launch_pass(medyan_mech* h, int which);
 // Host coordinates/forces (caller's bead order) to and from internal device
 // arrays; stream-ordered on s (the host buffer must stay valid until s syncs).
 cudaError_t coords_to_device(medyan_mech* h, const double* host, double* dev, cudaStream_t s);
-// The same through the handle's pinned staging, where staged(h, host) says
-// so, and the way out by plain copies; both ways out wait for the handle's
-// stream and hand out its force status (unless status is null).
-bool staged(medyan_mech* h, const double* host);
+// The same through the handle's pinned staging, where staged(h, host, most) says
+// so (networks of up to `most` beads, a kStage constant), and the way out by plain
+// copies; both ways out wait for the handle's stream and hand out its force
+// status (unless status is null).
+bool staged(medyan_mech* h, const double* host, int most);
 cudaError_t staged_in(medyan_mech* h, const double* host, double* dev);
 struct HostCopy {
     const double* dev;
     double* host;
 };
 cudaError_t staged_out(medyan_mech* h, const HostCopy* c, int n, bool energies, int* status);
+// Ahead of a plain copy: has an output's pages in memory while the device works.
+void populate_output(const medyan_mech* h, const double* host);
 cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
 // A minimization in two halves (cg.cu): enqueue everything on the handle's
 // stream, then wait and copy the results out.

@@ -43,3 +43,29 @@ def test_bead_order_costs_little(gpu_lib):
             ff.vectorize_all_force_fields(sv)
             t.append(best(lambda: ff.evaluate(x)))
     assert t[1] <= 1.15 * t[0], t
+
+
+def test_large_arrays_take_the_copies_time(gpu_lib):
+    """126,000 beads: coordinates alone took 1.7 times the plain copy through the
+    staging, an evaluation 1.6 times the two copies and the pass; 1.05 and 1.1
+    without it."""
+    import torch
+
+    n = 126000
+    sv, x = chain(n, False)
+    host, dev, back = torch.from_numpy(x), torch.empty(3 * n, dtype=torch.float64, device="cuda"), torch.empty(3 * n, dtype=torch.float64)
+
+    def copy_in():
+        dev.copy_(host)
+        torch.cuda.synchronize()
+
+    def copy_out():
+        back.copy_(dev)
+        torch.cuda.synchronize()
+
+    with ForceFieldManager("fp64") as ff:
+        ff.vectorize_all_force_fields(sv)
+        t_in, t_out = best(copy_in), best(copy_out)
+        t_set, t_eval = best(lambda: ff.set_coords(x)), best(lambda: ff.evaluate(x))
+    assert t_set <= 1.35 * t_in, (t_set, t_in)
+    assert t_eval <= 1.35 * (t_in + t_out), (t_eval, t_in, t_out)
