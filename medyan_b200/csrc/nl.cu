@@ -37,6 +37,8 @@ constexpr int kScanThreads = 256, kScanPer = 8, kScanShift = 11;
 constexpr int kScanTile = 1 << kScanShift;
 static_assert(kScanTile == kScanThreads * kScanPer, "a thread scans kScanPer counts");
 constexpr int kFound = 16;  // neighbors of a key that counting keeps for the writing
+constexpr int kLaneBin = 4; // cylinders of a bin that one lane takes (walk_key)
+constexpr int kKeyLanes = 4;  // threads that write a key's records
 
 struct Grid {
     double bin;
@@ -233,11 +235,16 @@ __global__ void k_fill_bins(CylDev c, const int* __restrict__ cell, const int* _
     }
 }
 
-// Neighbors of key i, found by a warp with a lane per bin of its stencil: the
-// bins hold a tenth of a cylinder on average, so one thread per key spent its
-// time on 27 dependent loads in a row (40,000 cylinders: 48 us; a warp 19). A key's pairs
-// are in bin order, dx outermost, then the bin's order. put(k, j): neighbor
-// number k of the key is j; returns their number. All 32 lanes call.
+// Neighbors of key i, found by a warp whose lanes read the 27 bins of the stencil
+// side by side: the bins hold a tenth of a cylinder on average, so one thread per
+// key spent its time on 27 dependent loads in a row (40,000 cylinders: 48 us; a
+// warp 19). Then each lane takes a bin's cylinders, or, where a bin holds more
+// than kLaneBin, all lanes take the bins' cylinders one after another, 32 at a
+// time: in a bundle a few bins hold all of them (rebuild of 2,000 cylinders with
+// 35,500 pairs: a lane per bin 510 us, now KEY_NOW; 400,000 spread cylinders: a
+// lane per bin 273 us, all lanes 302). A key's pairs are in bin order, dx
+// outermost, then the bin's order, either way. put(k, j): neighbor number k of the
+// key is j; returns their number. All 32 lanes call.
 template <class Put>
 __device__ __forceinline__ int walk_key(const CylDev& c, const Grid& G, int ci, int i, const Scan& start,
                                         const Item* __restrict__ items, const double* __restrict__ mid, double rmaxsq,
@@ -265,24 +272,46 @@ __device__ __forceinline__ int walk_key(const CylDev& c, const Grid& G, int ci, 
         if (d2 > rmaxsq || d2 < rminsq) return false;
         return !(skip_branch && c.branching[o.cyl] == i);
     };
-    int n = 0;
-    for (int q = q0; q < q1; ++q) n += is_pair(items[q]) ? 1 : 0;
-    if (!__any_sync(0xffffffffu, n)) return 0;
-    int before = n;  // pairs of the bins before this lane's
+    // v of the lanes up to this one
+    auto upto = [&](int v) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, before, o);
-        if (lane >= o) before += v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        return v;
+    };
+    if (!__any_sync(0xffffffffu, q1 - q0 > kLaneBin)) {
+        int n = 0;
+        for (int q = q0; q < q1; ++q) n += is_pair(items[q]) ? 1 : 0;
+        if (!__any_sync(0xffffffffu, n)) return 0;
+        int before = upto(n);  // pairs of the bins before this lane's
+        const int total = __shfl_sync(0xffffffffu, before, 31);
+        before -= n;
+        for (int q = q0; q < q1 && n > 0; ++q) {
+            if (!is_pair(items[q])) continue;
+            put(before, items[q].cyl);
+            ++before;
+            --n;
+        }
+        return total;
     }
-    const int total = __shfl_sync(0xffffffffu, before, 31);
-    before -= n;
-    for (int q = q0; q < q1 && n > 0; ++q) {
-        if (!is_pair(items[q])) continue;
-        put(before, items[q].cyl);
-        ++before;
-        --n;
+    const int end = upto(q1 - q0);  // cylinders of the bins up to this lane's
+    const int total = __shfl_sync(0xffffffffu, end, 31), base = q1 - end;
+    int found = 0;
+    for (int t0 = 0; t0 < total; t0 += 32) {
+        const int t = t0 + lane;
+        int b = 0;  // the bin of number t: the bins that end at or before it
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (__shfl_sync(0xffffffffu, end, b + s - 1) <= t) b += s;
+        const int q = __shfl_sync(0xffffffffu, base, b) + t;
+        const int j = t < total && is_pair(items[q]) ? items[q].cyl : -1;
+        const unsigned hits = __ballot_sync(0xffffffffu, j >= 0);
+        if (j >= 0) put(found + __popc(hits & ((1u << lane) - 1u)), j);
+        found += __popc(hits);
     }
-    return total;
+    return found;
 }
 
 // Counts the pairs of each key, a warp per key, and keeps its first neighbors.
@@ -319,18 +348,21 @@ struct Records {
     int* totals;
 };
 
-// Writes them: thread t < n the pairs of key t from what counting found (all
-// again by the warp when it found more than it kept), thread n + p n + i the
-// terms of plane p and cylinder i.
+// Writes them: kKeyLanes threads per key its pairs, from what counting found (all
+// again by the warp when it found more than it kept: with a thread per key a
+// warp walked 32 such keys one after another, half the time of a bundle's rebuild),
+// then a thread per plane p and cylinder i its terms.
 template <bool PAIRS>
 __global__ void __launch_bounds__(256) k_write_records(CylDev c, Grid G, BoundaryDev B, const double* __restrict__ mid,
                                                        const int* __restrict__ cell, Scan start,
                                                        const Item* __restrict__ items, double rmaxsq, double rminsq,
                                                        int skip_branch, Scan off, const int* __restrict__ found,
                                                        const int* __restrict__ err, Records R) {
-    const int m = c.n * (1 + B.n_planes), t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m = c.n * (1 + B.n_planes), u = blockIdx.x * blockDim.x + threadIdx.x, sub = u % kKeyLanes;
+    const bool key = u < kKeyLanes * c.n;
+    const int t = key ? u / kKeyLanes : u - (kKeyLanes - 1) * c.n;  // the count's index
     const int n_pairs = off[c.n], n_terms = off[m] - n_pairs, bad = *err;
-    if (t == 0 && R.totals) {
+    if (u == 0 && R.totals) {
         R.totals[0] = n_pairs;
         R.totals[1] = bad;
         R.totals[2] = n_terms;
@@ -347,17 +379,17 @@ __global__ void __launch_bounds__(256) k_write_records(CylDev c, Grid G, Boundar
             R.ex_krs[at] = k * c.eqlen[i] * c.eqlen[j];
         }
     };
-    if (t < c.n && n <= kFound)
-        for (int k = 0; k < n; ++k) put(t, o + k, found[(size_t)t * kFound + k]);
-    unsigned many = __ballot_sync(0xffffffffu, t < c.n && n > kFound);
+    if (key && n <= kFound)
+        for (int k = sub; k < n; k += kKeyLanes) put(t, o + k, found[(size_t)t * kFound + k]);
+    unsigned many = __ballot_sync(0xffffffffu, key && sub == 0 && n > kFound);
     for (; many; many &= many - 1u) {
         const int l = __ffs(many) - 1, i = __shfl_sync(0xffffffffu, t, l), at = __shfl_sync(0xffffffffu, o, l);
         walk_key(c, G, cell[i], i, start, items, mid, rmaxsq, rminsq, skip_branch,
                  [&](int k, int j) { put(i, at + k, j); });
     }
     if constexpr (!PAIRS) {
-        if (t < B.n_planes) R.planes[t] = B.planes[t];
-        if (t < c.n || n == 0) return;
+        if (u < B.n_planes) R.planes[u] = B.planes[u];
+        if (key || n == 0) return;
         const int p = t / c.n - 1, i = t % c.n;
         int at = o - n_pairs;
         if (n == 2) {
@@ -541,7 +573,7 @@ struct NLBuilder {
     cudaError_t enqueue_write(int skip_branch, const Records& R, cudaStream_t s) {
         const BoundaryDev B = boundary(!PAIRS);
         const float rmaxsq = nl.rmax * nl.rmax, rminsq = nl.rmin * nl.rmin;
-        const long long threads = (long long)n * (1 + B.n_planes);  // at least one block copies the planes
+        const long long threads = (long long)n * (kKeyLanes + B.n_planes);  // at least one block copies the planes
         k_write_records<PAIRS><<<blocks_of(threads > B.n_planes ? threads : B.n_planes + 1), 256, 0, s>>>(
             view(), make_grid(nl), B, mid.raw(), cell.raw(), starts(), items.raw(), (double)rmaxsq, (double)rminsq,
             skip_branch, offsets(), found.raw(), error(), R);
