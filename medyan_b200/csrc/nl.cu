@@ -241,8 +241,8 @@ __global__ void k_fill_bins(CylDev c, const int* __restrict__ cell, const int* _
 // warp 19). Then each lane takes a bin's cylinders, or, where a bin holds more
 // than kLaneBin, all lanes take the bins' cylinders one after another, 32 at a
 // time: in a bundle a few bins hold all of them (rebuild of 2,000 cylinders with
-// 35,500 pairs: a lane per bin 510 us, now KEY_NOW; 400,000 spread cylinders: a
-// lane per bin 273 us, all lanes 302). A key's pairs are in bin order, dx
+// 35,500 pairs: a lane per bin 510 us, now 147; 400,000 spread cylinders: a
+// lane per bin 271 us, all lanes 302). A key's pairs are in bin order, dx
 // outermost, then the bin's order, either way. put(k, j): neighbor number k of the
 // key is j; returns their number. All 32 lanes call.
 template <class Put>
