@@ -421,7 +421,6 @@ static bool make_staging(medyan_mech* h) {
 // managed) takes plain copies, which need no host time there, as does everything
 // when no staging is to be had.
 bool staged(medyan_mech* h, const double* host, int most) {
-    if (most == kStageIn && h->n_beads < kStageInLeast && h->identity_order) return false;
     cudaPointerAttributes a;
     return h->n_beads > 0 && h->n_beads <= most && cudaSetDevice(h->device) == cudaSuccess &&
            cudaPointerGetAttributes(&a, host) == cudaSuccess && a.type == cudaMemoryTypeUnregistered && make_staging(h);
@@ -740,8 +739,7 @@ medyan_status medyan_mech_set_coords(medyan_mech* h, const double* coord) {
     if (!h || (!coord && h->n_beads)) return MEDYAN_ERR_INVALID_ARG;
     // what follows this call uses it: not in the first evaluation's time
     if (h->n_beads > 0 && h->n_beads <= kStageMinimize && cudaSetDevice(h->device) == cudaSuccess) make_staging(h);
-    cudaError_t e = staged(h, coord, kStageIn) ? staged_in(h, coord, h->x.raw())
-                                               : coords_to_device(h, coord, h->x.raw(), h->stream);
+    cudaError_t e = coords_to_device(h, coord, h->x.raw(), h->stream);
     if (e != cudaSuccess) return cuda_status(e);
     return sync_status(h);
 }

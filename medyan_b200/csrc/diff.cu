@@ -346,7 +346,7 @@ int blocks_for(int n) {
 }
 
 // Uploads v (caller's order) into h->hv_v (internal order).
-// most: what the call stages (kStageIn, or kStageBoth with a result of the same size)
+// most: the largest network whose direction is staged (0: none)
 cudaError_t upload_direction(medyan_mech* h, const double* v, int most) {
     const int n3 = 3 * h->n_beads;
     cudaError_t e = h->hv_v.reserve(n3 ? n3 : 1);
@@ -385,7 +385,7 @@ extern "C" medyan_status medyan_mech_param_grad(medyan_mech* h, int32_t ff, cons
     DevBuf<double>& gp = h->pg_p;
     cudaError_t ce = gk.reserve(count);
     if (ce == cudaSuccess) ce = gp.reserve(count);
-    if (ce == cudaSuccess && v) ce = upload_direction(h, v, kStageIn);
+    if (ce == cudaSuccess && v) ce = upload_direction(h, v, 0);
     if (ce != cudaSuccess) return cuda_status(ce);
     const double* dv = v ? h->hv_v.raw() : nullptr;
     const int g = (count + kThreads - 1) / kThreads;

@@ -24,16 +24,15 @@ constexpr int kIoSlots = 4;  // pieces of the staging of host coordinates
 // saves the copies' fixed cost, but one host thread fills it at 12 GB/s, where
 // the driver copies pageable memory at 20. Staged and plain, us, results in memory
 // that is in use:
-//   coordinates in: 85 beads 16.7 and 13.8 (in chain order, else 16.3 and 19.3), 550
-//     17.4 and 19.2, 2,700 beads 21.6 and 47.4, 5,400 25.4 and 22.5, 42,000 90 and
-//     71, 420,000 900 and 514 (the driver's copies up to 64 KB take another way)
 //   forces out: 30,000 82 and 90, 42,000 105 and 107, 60,000 154 and 133
 //   both (evaluate): 21,000 105 and 120, 27,000 134 and 135, 33,000 163 and 156,
 //     60,000 277 and 235, 420,000 1,822 and 1,070 (Hessian-vector products alike)
 //   minimization, 8 energy calls: 60,000 675 and 737, 84,000 712 and 641, 126,000
 //     1,000 and 849, 420,000 3,061 and 2,263
-constexpr int kStageIn = 2730, kStageOut = 42000, kStageBoth = 30000, kStageMinimize = 72000;
-constexpr int kStageInLeast = 350;  // coordinates in, in chain order
+// Coordinates alone always take the plain copy: staged and plain, 504 beads 19.1 and
+// 15.5, 1,050 20.7 and 17.3, 2,600 23.4 and 21.6, 42,000 90 and 71 (in another order
+// than the chains' 504 18.9 and 18.2, 2,600 23.0 and 24.0).
+constexpr int kStageOut = 42000, kStageBoth = 30000, kStageMinimize = 72000;
 
 template <class T>
 struct DevBuf {

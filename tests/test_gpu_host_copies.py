@@ -69,3 +69,15 @@ def test_large_arrays_take_the_copies_time(gpu_lib):
         t_set, t_eval = best(lambda: ff.set_coords(x)), best(lambda: ff.evaluate(x))
     assert t_set <= 1.35 * t_in, (t_set, t_in)
     assert t_eval <= 1.35 * (t_in + t_out), (t_eval, t_in, t_out)
+
+
+def test_coordinates_alone_cost_no_launch(gpu_lib):
+    """Through the staging, 504 beads took 1.25 times as long as 312, which took
+    the plain copy; 1.03 when both do."""
+    t = []
+    for n in (312, 504):
+        sv, x = chain(n, False)
+        with ForceFieldManager("fp64") as ff:
+            ff.vectorize_all_force_fields(sv)
+            t.append(best(lambda: ff.set_coords(x), reps=1000))
+    assert t[1] <= 1.13 * t[0], t
