@@ -720,8 +720,10 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     const int n3 = 3 * h->n_beads;
     cudaStream_t s = h->stream;
     h->cg_params = *p;
-    h->cg_team = loop_team(h->chain, h->ff);
     cudaError_t e = cudaSetDevice(h->device);
+    if (e == cudaSuccess) e = init_cg_loop(h->loop_room);
+    if (e != cudaSuccess) return cuda_status(e);
+    h->cg_team = loop_team(h->chain, h->ff, h->loop_room);
     if (e == cudaSuccess) e = h->cg_dir.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess) e = h->cg_force2.reserve(n3 ? n3 : 1);
     if (e == cudaSuccess) e = h->cg_min_coords.reserve(n3 ? n3 : 1);
@@ -732,7 +734,6 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     if (e == cudaSuccess && h->cg_team > 0)
         e = h->cg_rows.reserve(loop_erow_doubles(loop_row_count(h->chain, h->ff)) + loop_vrow_doubles(vec_blocks(n3)));
     if (e == cudaSuccess && h->cg_team > 0) e = h->cg_words.reserve(kLoopWords);
-    if (e == cudaSuccess && h->cg_team > 0) e = init_cg_loop();
     if (e != cudaSuccess) return cuda_status(e);
     const CGLaunch c = make_launch(h);
     e = staged(h, coord_in, kStageMinimize) ? staged_in(h, coord_in, c.x) : coords_to_device(h, coord_in, c.x, s);
@@ -1043,6 +1044,15 @@ medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p)
 }
 
 }  // namespace mb
+
+// For tests, not part of the interface: the room on the device that the handle's
+// minimizations go by. 0, 0: they run in the graph loop, a batch with this replica packed.
+extern "C" medyan_status medyan_internal_loop_room(medyan_mech* h, int32_t cluster, int32_t grid) {
+    if (!h || cluster < 0 || grid < 0) return MEDYAN_ERR_INVALID_ARG;
+    h->loop_room.cluster = cluster;
+    h->loop_room.grid = grid;
+    return MEDYAN_OK;
+}
 
 extern "C" medyan_status medyan_cg_minimize(medyan_mech* h, const medyan_cg_params* p, double* coord_inout,
                                             double* force_out, medyan_min_result* out) {

@@ -14,8 +14,9 @@ namespace mb {
 // A cluster's barrier takes 0.7 us where the grid's takes 1.2, so teams of up
 // to 16 blocks (the largest cluster) are clusters. The graph loop takes over
 // where its kernels, which hold three to four times as many threads per SM,
-// are faster.
-int loop_team(const ChainDev& ch, const DeviceFF& ff) {
+// are faster, and where the device does not hold the team at once (fewer SMs): a
+// launch would be refused.
+int loop_team(const ChainDev& ch, const DeviceFF& ff, const LoopRoom& room) {
     if (ch.n_pos <= 0 || ch.n_pos > kLoopBeads) return 0;
     auto chunks = [](int n, int per) { return (n + per - 1) / per; };
     const int tasks = chunks(ff.n_excl, 8) + chunks(ff.n_branch, 32) + chunks(ff.n_stretch, 32) + chunks(ff.n_bend, 32) +
@@ -26,7 +27,8 @@ int loop_team(const ChainDev& ch, const DeviceFF& ff) {
     const int blocks = chunks(tasks, kWarps) + rows;
     int team = 1;
     while (team < blocks && team < kLoopCluster) team *= 2;
-    return blocks <= kLoopCluster ? team : (blocks < kLoopGrid ? blocks : kLoopGrid);
+    if (blocks > kLoopCluster) team = blocks < kLoopGrid ? blocks : kLoopGrid;
+    return team <= (blocks > kLoopCluster ? room.grid : room.cluster) ? team : 0;
 }
 
 int loop_row_count(const ChainDev& ch, const DeviceFF& ff) {
@@ -37,19 +39,25 @@ int loop_row_count(const ChainDev& ch, const DeviceFF& ff) {
 
 size_t loop_erow_doubles(int rows) { return 2 * (size_t)kMaxLambda * kRowVals * rows; }
 
-cudaError_t init_cg_loop() {
+cudaError_t init_cg_loop(LoopRoom& room) {
     static std::mutex mu;
-    static bool done[64];
+    static LoopRoom rooms[64];
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> lock(mu);
-    if (done[dev]) return cudaSuccess;
-    e = allow_clusters<false>();
-    if (e == cudaSuccess) e = init_cg_loop_wide();
-    if (e == cudaSuccess) done[dev] = true;
-    return e;
+    if (rooms[dev].grid < 0) {
+        LoopRoom r;
+        r.cluster = kLoopCluster;
+        r.grid = kLoopGrid;
+        e = init_kernels<false>(r);
+        if (e == cudaSuccess) e = init_cg_loop_wide(r);
+        if (e != cudaSuccess) return e;
+        rooms[dev] = r;
+    }
+    if (room.grid < 0) room = rooms[dev];
+    return cudaSuccess;
 }
 
 cudaError_t launch_cg_loop(const LoopArgs& a, int prec, int team, cudaStream_t s) {

@@ -40,18 +40,19 @@ constexpr int kLoopBeads = 350000;  // larger networks run in the graph loop
 constexpr int kLoopWideBeads = 75000;  // larger ones take blocks of 512 threads
 
 // Blocks of a team for this network, 0 when the network is better off in the
-// graph loop.
-int loop_team(const ChainDev& ch, const DeviceFF& ff);
+// graph loop, or the device has no room for the team.
+int loop_team(const ChainDev& ch, const DeviceFF& ff, const LoopRoom& room);
 // Energy rows of a pass at one step size, and the doubles that the rows and the
 // vector passes' sums take.
 int loop_row_count(const ChainDev& ch, const DeviceFF& ff);
 size_t loop_erow_doubles(int rows);
 __host__ __device__ __forceinline__ size_t loop_vrow_doubles(int vb) { return 2 * (size_t)(vb == 1 ? 8 : vb) * 4; }
 // Kernel attributes, once per device (the current one); before the first launch.
-cudaError_t init_cg_loop();
+// room: what the device holds, unless it is set already.
+cudaError_t init_cg_loop(LoopRoom& room);
 cudaError_t launch_cg_loop(const LoopArgs& a, int prec, int team, cudaStream_t s);
 // its parts on blocks of 512 threads (cg_loop_wide.cu)
-cudaError_t init_cg_loop_wide();
+cudaError_t init_cg_loop_wide(LoopRoom& room);
 cudaError_t launch_cg_loop_wide(const LoopArgs& a, int prec, int team, cudaStream_t s);
 
 

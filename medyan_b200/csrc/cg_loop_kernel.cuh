@@ -935,21 +935,55 @@ cudaError_t launch(const LoopArgs& a, int team, cudaStream_t s) {
     return cudaLaunchKernelEx(&c, k_cg_loop<R, FIXED, false>, a);
 }
 
+// A kernel's attributes, and the room for it: the largest cluster, or the blocks
+// of a cooperative grid.
+template <class Kernel>
+cudaError_t init_kernel(Kernel k, bool cluster, LoopRoom& room) {
+    if (!cluster) {
+        int dev = 0, sms = 0, coop = 0, per = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kLoopThreads, sizeof(Smem));
+        if (e == cudaSuccess && room.grid > (coop ? per * sms : 0)) room.grid = coop ? per * sms : 0;
+        return e;
+    }
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(kLoopCluster);
+    c.blockDim = dim3(kLoopThreads);
+    c.dynamicSmemBytes = sizeof(Smem);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kLoopCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &c) != cudaSuccess) {
+        cudaGetLastError();  // no such cluster on this device
+        n = 0;
+    }
+    if (n < 1) room.cluster = 0;
+    return cudaSuccess;
+}
+
 // BATCH: the kernels that take a batch's replicas too.
 template <bool BATCH, class R, bool FIXED>
-cudaError_t allow_clusters_of() {
-    cudaError_t e = cudaFuncSetAttribute(k_cg_loop<R, FIXED, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+cudaError_t init_kernels_of(LoopRoom& room) {
+    cudaError_t e = init_kernel(k_cg_loop<R, FIXED, true>, true, room);
+    if (e == cudaSuccess) e = init_kernel(k_cg_loop<R, FIXED, false>, false, room);
     if constexpr (BATCH)
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_cg_loop_batch<R, FIXED>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = init_kernel(k_cg_loop_batch<R, FIXED>, true, room);
     return e;
 }
 template <bool BATCH>
-cudaError_t allow_clusters() {
-    cudaError_t e = allow_clusters_of<BATCH, float, false>();
-    if (e == cudaSuccess) e = allow_clusters_of<BATCH, float, true>();
-    if (e == cudaSuccess) e = allow_clusters_of<BATCH, double, false>();
-    if (e == cudaSuccess) e = allow_clusters_of<BATCH, double, true>();
+cudaError_t init_kernels(LoopRoom& room) {
+    cudaError_t e = init_kernels_of<BATCH, float, false>(room);
+    if (e == cudaSuccess) e = init_kernels_of<BATCH, float, true>(room);
+    if (e == cudaSuccess) e = init_kernels_of<BATCH, double, false>(room);
+    if (e == cudaSuccess) e = init_kernels_of<BATCH, double, true>(room);
     return e;
 }
 

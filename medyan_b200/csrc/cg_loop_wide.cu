@@ -5,7 +5,7 @@
 
 namespace mb {
 
-cudaError_t init_cg_loop_wide() { return allow_clusters<true>(); }
+cudaError_t init_cg_loop_wide(LoopRoom& room) { return init_kernels<true>(room); }
 
 cudaError_t launch_cg_loop_wide(const LoopArgs& a, int prec, int team, cudaStream_t s) {
     return launch_single(a, prec, team, s);

@@ -18,6 +18,11 @@
 namespace mb {
 
 struct medyan_async;  // async.cu
+// What the device holds at once of the resident minimizer loop (cg_loop.cu):
+// blocks of a cluster, blocks of a cooperative grid; -1: not asked yet.
+struct LoopRoom {
+    int cluster = -1, grid = -1;
+};
 constexpr int kIoSlots = 4;  // pieces of the staging of host coordinates
 // Largest networks (beads) whose host arrays go through the staging, by what the
 // call moves; larger ones take plain copies. Two things meet here: the staging
@@ -230,6 +235,7 @@ struct medyan_mech {
     mb::DevBuf<double> cg_rows;
     mb::DevBuf<int> cg_words;
     int cg_team = 0;
+    mb::LoopRoom loop_room;
     medyan_cg_params cg_params{};
     cudaGraphExec_t cg_graph = nullptr;   // instantiated minimization graph
     // pinned area for the per-call results the host reads back and a

@@ -302,8 +302,11 @@ medyan_status pack_batch(PackedBatch& pb, const std::vector<medyan_mech*>& h) {
 
 // ------------------------------------------------------------ resident loop
 bool batch_loop_takes(const std::vector<medyan_mech*>& h) {
-    for (const auto* m : h)
-        if (m->n_beads <= 0 || m->n_beads > kLoopBatchBeads || loop_team(m->chain, m->ff) == 0) return false;
+    const LoopRoom largest{kLoopCluster, kLoopGrid};  // only the room for a cluster counts
+    for (auto* m : h)
+        if (m->n_beads <= 0 || m->n_beads > kLoopBatchBeads || init_cg_loop(m->loop_room) != cudaSuccess ||
+            m->loop_room.cluster < kLoopCluster || loop_team(m->chain, m->ff, largest) == 0)
+            return false;
     return true;
 }
 
@@ -324,7 +327,7 @@ medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h
         if (mask < 0) mask = m->ff.branch_mask;
         else if (mask != m->ff.branch_mask) return MEDYAN_ERR_UNSUPPORTED;
     }
-    cudaError_t e = init_cg_loop();
+    cudaError_t e = cudaSuccess;
     for (auto* m : h)  // their records are complete
         if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     cudaStream_t s = pb.stream;
