@@ -242,6 +242,23 @@ medyan_status upload_system(medyan_mech* h, const medyan_system* s) {
     return refresh_device_ff(h);
 }
 
+// The block table and the energy rows that the launch shapes make.
+void energy_rows(const ChainDev& ch, DeviceFF& ff, EnergyScratch& es) {
+    const int counts[6] = {ff.n_stretch, ff.n_bend, ff.n_linker, ff.n_motor, ff.n_branch, ff.n_boundary};
+    ff.seg[0] = 0;
+    const int bb = bonded_block_of(ff);
+    for (int q = 0; q < 6; ++q) ff.seg[q + 1] = ff.seg[q] + (counts[q] + bb - 1) / bb;
+    es.n_blocks_chain = ch.n_pos > 0 ? chain_blocks(ch) : 0;
+    es.n_blocks_bonded = ff.seg[6];
+    es.n_blocks_excl = excl_blocks(ff);
+}
+
+DefaultShapes::DefaultShapes(const medyan_mech* h) : ch(h->chain), ff(h->ff), es(h->es) {
+    ff.bonded_block = ff.excl_block = 0;
+    ch.energy_blocks_per_sm = 0;
+    energy_rows(ch, ff, es);
+}
+
 // Re-derives DeviceFF pointers and the block table from the owned buffers,
 // and sizes the energy scratch.
 medyan_status refresh_device_ff(medyan_mech* h) {
@@ -266,14 +283,10 @@ medyan_status refresh_device_ff(medyan_mech* h) {
     h->chain.flags = h->chain_flags.raw();
     h->chain.link_p = h->chain_link_p.raw();
     h->chain.bend_p = h->chain_bend_p.raw();
-    const int counts[6] = {ff.n_stretch, ff.n_bend, ff.n_linker, ff.n_motor, ff.n_branch, ff.n_boundary};
-    ff.seg[0] = 0;
-    const int bb = bonded_block_of(ff);
-    for (int q = 0; q < 6; ++q) ff.seg[q + 1] = ff.seg[q] + (counts[q] + bb - 1) / bb;
-    h->es.n_blocks_chain = h->chain.n_pos > 0 ? chain_blocks(h->chain) : 0;
-    h->es.n_blocks_bonded = ff.seg[6];
-    h->es.n_blocks_excl = excl_blocks(ff);
-    const size_t need = (size_t)kMaxLambda * (h->es.total() + 1) * 4;
+    energy_rows(h->chain, ff, h->es);
+    DefaultShapes d(h);  // what finishes a resident loop's minimization
+    const size_t rows = h->es.total() > d.es.total() ? h->es.total() : d.es.total();
+    const size_t need = (size_t)kMaxLambda * (rows + 1) * 4;
     cudaError_t e = h->partial.reserve(need);
     {
         // fused-pass scratch; the group tickets start at zero (stream-ordered

@@ -462,6 +462,11 @@ namespace {
 struct CGLaunch {
     medyan_mech* h;
     int n3, vb;
+    // energies: in the handle's launch shapes, or the default ones where the
+    // resident loop, which adds in their order, has begun the minimization
+    ChainDev ch;
+    DeviceFF ff;
+    EnergyScratch es;
     double *x, *d, *f0, *f1, *part, *minE;
     CGState* st;
     LambdaSet* L;
@@ -475,6 +480,15 @@ CGLaunch make_launch(medyan_mech* h) {
     c.h = h;
     c.n3 = 3 * h->n_beads;
     c.vb = vec_blocks(c.n3);
+    c.ch = h->chain;
+    c.ff = h->ff;
+    c.es = h->es;
+    if (h->cg_team > 0) {
+        const DefaultShapes s(h);
+        c.ch = s.ch;
+        c.ff = s.ff;
+        c.es = s.es;
+    }
     c.x = h->x.raw();
     c.d = h->cg_dir.raw();
     c.f0 = h->f.raw();
@@ -495,7 +509,7 @@ CGLaunch make_launch(medyan_mech* h) {
 // search, the forces at its first trial step.
 void enqueue_ls_pass(const CGLaunch& c, cudaStream_t s, cudaGraphConditionalHandle h_ls,
                      cudaGraphConditionalHandle h_force) {
-    launch_evaluate(c.h->chain, c.h->ff, c.h->prec, c.x, c.d, c.L, c.spec, c.h->es, c.spec_fs, s, &c.h->fork);
+    launch_evaluate(c.ch, c.ff, c.h->prec, c.x, c.d, c.L, c.spec, c.es, c.spec_fs, s, &c.h->fork);
     k_ls_decide<<<1, 1, 0, s>>>(c.st, c.L, c.h->energy_out.raw(), c.h->fs.status, h_ls, h_force);
 }
 
@@ -654,13 +668,19 @@ static cudaError_t cg_start(medyan_mech* h, const CGLaunch& c, cudaStream_t s) {
     return e;
 }
 
+static void cg_energy(const CGLaunch& c, cudaStream_t s) {
+    launch_energy(c.ch, c.ff, c.h->prec, c.x, nullptr, c.h->lam_zero.raw(), c.es, s, &c.h->fork);
+}
+
 // The iteration loop as one graph launch (from the state on the device), the
 // epilogue and energiesAfter.
 static cudaError_t cg_graph_loop(medyan_mech* h, const CGLaunch& c, cudaStream_t s) {
     cudaError_t e = cudaSuccess;
     // the graph captures the force-field records by value: rebuild it after
     // any re-vectorization (generation counter) or precision change
-    if (h->cg_graph && (h->cg_graph_gen != h->ff_gen || h->cg_graph_prec != h->prec)) {
+    const bool shapes = h->cg_team > 0;
+    if (h->cg_graph &&
+        (h->cg_graph_gen != h->ff_gen || h->cg_graph_prec != h->prec || h->cg_graph_default != shapes)) {
         cudaGraphExecDestroy(h->cg_graph);
         h->cg_graph = nullptr;
     }
@@ -669,11 +689,12 @@ static cudaError_t cg_graph_loop(medyan_mech* h, const CGLaunch& c, cudaStream_t
         if (e != cudaSuccess) return e;
         h->cg_graph_gen = h->ff_gen;
         h->cg_graph_prec = h->prec;
+        h->cg_graph_default = shapes;
     }
     e = cudaGraphLaunch(h->cg_graph, s);
     if (e != cudaSuccess) return e;
     k_cg_finalize<<<c.vb, kVecThreads, 0, s>>>(c.n3, c.x, c.minE, c.f0, c.f1, c.st);
-    enqueue_energy(h, c.x, nullptr, h->lam_zero.raw(), s);
+    cg_energy(c, s);
     k_cg_record_final<<<1, 1, 0, s>>>(c.st, h->energy_out.raw(), h->cg_eout.raw() + kOut);
     return cudaGetLastError();
 }
@@ -681,7 +702,7 @@ static cudaError_t cg_graph_loop(medyan_mech* h, const CGLaunch& c, cudaStream_t
 // A whole minimization in the graph loop: energiesBefore, the first force
 // (parity 1 -> f0), F.F, d = F, then the loop.
 static cudaError_t cg_graph_run(medyan_mech* h, const CGLaunch& c, cudaStream_t s) {
-    enqueue_energy(h, c.x, nullptr, h->lam_zero.raw(), s);
+    cg_energy(c, s);
     k_cg_record_energy<<<1, 1, 0, s>>>(c.st, h->energy_out.raw(), h->cg_eout.raw(), 1);
     enqueue_step(c, s);
     return cg_graph_loop(h, c, s);

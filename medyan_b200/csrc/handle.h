@@ -254,6 +254,7 @@ struct medyan_mech {
     double* io = nullptr;
     cudaEvent_t io_done[mb::kIoSlots] = {};
     int cg_graph_prec = -1;
+    bool cg_graph_default = false;        // captured with the default launch shapes
     long long cg_graph_gen = -1;          // ff_gen the graph was captured with
     long long ff_gen = 0;                 // bumped whenever DeviceFF changes
 
@@ -304,6 +305,15 @@ cudaError_t staged_out(medyan_mech* h, const HostCopy* c, int n, bool energies, 
 // Ahead of a plain copy: has an output's pages in memory while the device works.
 void populate_output(const medyan_mech* h, const double* host);
 cudaError_t plain_out(medyan_mech* h, const double* dev, double* host, bool energies, int* status);
+void energy_rows(const ChainDev& ch, DeviceFF& ff, EnergyScratch& es);
+// The handle's records in the default launch shapes, whose energy rows are the
+// resident loop's: a minimization that it hands over keeps the order of its sums.
+struct DefaultShapes {
+    ChainDev ch;
+    DeviceFF ff;
+    EnergyScratch es;
+    explicit DefaultShapes(const medyan_mech* h);
+};
 // A minimization in two halves (cg.cu): enqueue everything on the handle's
 // stream, then wait and copy the results out.
 medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double* coord_in);

@@ -1,0 +1,71 @@
+"""A minimization that the resident loop begins and another form finishes: a
+cylinder pair turns collinear at the line search's first trial, so the loop stops
+in front of that pass. Springs in powers of two bring the pair there exactly:
+two beads 2 t apart, force 64 * 2 t on each, first step size 2^-7."""
+import numpy as np
+import pytest
+
+from medyan_b200._abi import SystemView
+from medyan_b200.forcefield import ForceFieldManager, conjugate_gradient_params as cgp
+from medyan_b200.network import make_workload
+
+from .test_gpu_loop_room import counts, set_room
+
+pytestmark = pytest.mark.gpu
+
+T = 2.0 ** -10
+
+
+def system(n_fil, n_cyl, box, seed=11, turns=True):
+    """A network and, in front of its box, the pair (its repulsion too weak to move it)."""
+    net = make_workload(0, n_fil=n_fil, cyl_per_fil=n_cyl, box=box, n_linker=n_fil if n_fil > 20 else 0,
+                        n_branch=n_fil // 10, n_motor=0, seed=seed)
+    n = net.n_beads
+    x = (net.coords + np.random.default_rng(seed).normal(0.0, 0.1, net.coords.shape)).reshape(-1)
+    ff = dict(net.ff)
+    if not turns:
+        return SystemView(n, **ff), x
+    pair = np.array([[0, 0, 0], [8, 0, 0], [16, 0, 1], [32, T, 1], [32, T + 1, 1]], float) + [-512.0, 0.0, 0.0]
+    ff["stretch_beads"] = np.vstack([ff["stretch_beads"], [[3 * (n + 3), 3 * (n + 4)]]])
+    ff["stretch_k"], ff["stretch_l0"] = np.append(ff["stretch_k"], 64.0), np.append(ff["stretch_l0"], 1 + 2 * T)
+    ff.update(excl_beads=[[3 * n, 3 * (n + 1), 3 * (n + 2), 3 * (n + 3)]], excl_k=[1e-30], excl_eqlen=[[8.0, 16.0]])
+    return SystemView(n + 5, **ff), np.append(x, pair.reshape(-1))
+
+
+def params(limit=30, line_search="BACKTRACKING"):
+    return cgp(grad_tol=1e-9, energy_rel_tol=0.0, energy_call_limit=limit, max_dist=1e9, lambda_max=2.0 ** -7,
+               line_search=line_search)
+
+
+SHAPES = [{}, dict(bonded_threads=128, excl_threads=32, chain_energy_blocks_per_sm=2)]
+
+
+@pytest.mark.parametrize("size", [(4, 3, 700.0), (60, 10, 1800.0), (1500, 10, 4200.0)])
+@pytest.mark.parametrize("line_search", ["BACKTRACKING", "QUADRATIC"])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_handed_over_is_the_graph_loop(gpu_lib, oracle, size, line_search, precision):
+    """Bit for bit the graph loop's own run, in any launch shapes: the graph
+    loop goes on in the order of the resident loop's sums."""
+    sv, x = system(*size)
+    p = params(line_search=line_search)
+    with ForceFieldManager(precision) as ff:
+        ff.vectorize_all_force_fields(sv)
+        ff.set_deterministic(True)
+        ff.set_coords(x)
+        runs = []
+        for shapes in SHAPES:
+            if shapes:
+                ff.set_shapes(**shapes)
+            runs.append(ff.minimize(x, p))
+        ff.set_shapes(bonded_threads=256, excl_threads=64, chain_energy_blocks_per_sm=4)
+        set_room(ff.lib, ff.handle, 0, 0)
+        want = ff.minimize(x, p)
+    for s, xg, f, r in runs:
+        assert s == want[0] == 0 and counts(r) == counts(want[3]) and r.num_iter > 3
+        assert np.array_equal(xg, want[1]) and np.array_equal(f, want[2])
+        assert np.array_equal(np.array(r.energy_before), np.array(want[3].energy_before))
+        assert np.array_equal(np.array(r.energy_after), np.array(want[3].energy_after))
+    if precision == "fp64":
+        so, xo, fo, ro = oracle.minimize(sv, x, p)
+        assert so == 0 and counts(ro) == counts(want[3])
+        assert np.abs(xo - want[1]).max() <= (1e-7 if line_search == "BACKTRACKING" else 1e-6)
