@@ -8,8 +8,8 @@
 // - the resident loop (cg_loop_kernel.cuh): one kernel whose thread-block
 //   clusters take the replicas from a queue, the largest first, and minimize
 //   one each on its handle's own records. No replica waits for another;
-// - packed (pbatch.h), for batches with large replicas and for replicas that
-//   met a pair which needs a quadrature: the replicas' device arrays in one
+// - packed (pbatch.h), for batches with large replicas, and for replicas that met
+//   a pair which needs a quadrature, from where they met it: the replicas' device arrays in one
 //   set and one conjugate-gradient loop for all of them, every force and
 //   energy kernel launched once per pass. Its line-search loop runs until the
 //   slowest replica has accepted a step, about 300 us per iteration on an
@@ -23,6 +23,10 @@
 struct medyan_batch {
     std::vector<medyan_mech*> h;
     mb::PackedBatch pb;
+    // the replicas that the resident loop last left to the packed one, in the default
+    // shapes, whose sums are the resident loop's
+    mb::PackedBatch tail;
+    std::vector<int> tail_of;
     ~medyan_batch() {
         for (auto* p : h) medyan_mech_destroy(p);
     }
@@ -89,54 +93,65 @@ medyan_status medyan_batch_minimize(medyan_batch* b, const medyan_cg_params* p, 
     std::vector<CGState> sf(n);
     std::vector<double> eo((size_t)n * 2 * (MEDYAN_FF_COUNT + 1));
     int force_status = 0;
-    // one replica per cluster of the resident loop; replicas that it cannot
-    // finish, and batches that it does not take, run packed
+    // One replica per cluster of the resident loop. Replicas that it cannot finish go
+    // on packed, from where it left them; batches that it does not take run packed.
+    // Started again, in the batch's own packing, they took the whole run twice, and
+    // every such call packed and captured that packing again: one of 9 networks of
+    // 400 cylinders, 4 energy calls, 1,817 us, now 586 (packed from the start: 728).
     std::vector<int> rest;
-    if (batch_loop_takes(b->h)) {
+    std::vector<PackedCarry> carry;
+    const bool resident = batch_loop_takes(b->h);
+    if (resident) {
         std::vector<int> outcome(n, 0);
         const medyan_status st = batch_loop_run(pb, b->h, p, coords_inout, forces_out, sf.data(), eo.data(), outcome.data(),
                                                 &force_status);
         if (st != MEDYAN_OK) return st;
-        for (int r = 0; r < n; ++r)
-            if (outcome[r] != kLoopDone) rest.push_back(r);
+        for (int r = 0; r < n; ++r) {
+            if (outcome[r] == kLoopDone) continue;
+            if (outcome[r] == kLoopHandOver) carry.push_back(batch_loop_carry(pb, r, sf[r], (int)rest.size()));
+            rest.push_back(r);
+        }
     } else {
         for (int r = 0; r < n; ++r) rest.push_back(r);
     }
     if (!rest.empty()) {
         const int m = (int)rest.size();
+        PackedBatch& pk = resident ? b->tail : pb;
+        if (resident) {
+            pk.deterministic = pb.deterministic;
+            if (b->tail_of != rest) {
+                b->tail_of.clear();
+                pk.repack = true;
+                if (pk.graph) cudaGraphExecDestroy(pk.graph);
+                pk.graph = nullptr;
+            }
+        }
         std::vector<medyan_mech*> hs(m);
         for (int i = 0; i < m; ++i) hs[i] = b->h[rest[i]];
-        // another set of replicas than the last packing's: pack, and capture the loop, again
-        auto forget = [&] {
-            if (m == n) return;
-            pb.repack = true;
-            if (pb.graph) cudaGraphExecDestroy(pb.graph);
-            pb.graph = nullptr;
-        };
-        forget();
-        medyan_status st = pack_batch(pb, hs);
+        medyan_status st = pack_batch(pk, hs);
         if (st != MEDYAN_OK) return st;
-        cudaStream_t s = pb.stream;
+        if (resident) b->tail_of = rest;
+        cudaStream_t s = pk.stream;
         for (int i = 0; i < m; ++i) {
-            cudaError_t e = coords_to_device(hs[i], coords_inout[rest[i]], pb.x.raw() + 3 * (size_t)pb.base[i], s);
+            cudaError_t e = coords_to_device(hs[i], coords_inout[rest[i]], pk.x.raw() + 3 * (size_t)pk.base[i], s);
             if (e != cudaSuccess) return cuda_status(e);
         }
-        st = cg_batch_run(pb, hs[0]->prec, p);
+        st = cg_batch_run(pk, hs[0]->prec, p, carry);
         if (st != MEDYAN_OK) return st;
         std::vector<CGState> sp(m);
         std::vector<double> ep((size_t)m * 2 * (MEDYAN_FF_COUNT + 1));
-        cudaError_t e = cudaMemcpyAsync(sp.data(), pb.st.raw(), sizeof(CGState) * m, cudaMemcpyDeviceToHost, s);
+        cudaError_t e = cudaMemcpyAsync(sp.data(), pk.st.raw(), sizeof(CGState) * m, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(ep.data(), pb.eout.raw(), sizeof(double) * ep.size(), cudaMemcpyDeviceToHost, s);
+            e = cudaMemcpyAsync(ep.data(), pk.eout.raw(), sizeof(double) * ep.size(), cudaMemcpyDeviceToHost, s);
         for (int i = 0; i < m && e == cudaSuccess; ++i) {
-            const size_t o = 3 * (size_t)pb.base[i];
+            const size_t o = 3 * (size_t)pk.base[i];
             const int r = rest[i];
-            e = coords_to_host(hs[i], pb.x.raw() + o, coords_inout[r], s);
-            if (e == cudaSuccess && forces_out && forces_out[r]) e = coords_to_host(hs[i], pb.fcur.raw() + o, forces_out[r], s);
+            e = coords_to_host(hs[i], pk.x.raw() + o, coords_inout[r], s);
+            if (e == cudaSuccess && forces_out && forces_out[r]) e = coords_to_host(hs[i], pk.fcur.raw() + o, forces_out[r], s);
         }
         int status = 0;
-        if (e == cudaSuccess && pb.deterministic)
-            e = cudaMemcpyAsync(&status, pb.fs.status, sizeof(int), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && pk.deterministic)
+            e = cudaMemcpyAsync(&status, pk.fs.status, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return cuda_status(e);
         force_status |= status;
@@ -145,7 +160,6 @@ medyan_status medyan_batch_minimize(medyan_batch* b, const medyan_cg_params* p, 
             std::memcpy(eo.data() + (size_t)rest[i] * 2 * (MEDYAN_FF_COUNT + 1), ep.data() + (size_t)i * 2 * (MEDYAN_FF_COUNT + 1),
                         sizeof(double) * 2 * (MEDYAN_FF_COUNT + 1));
         }
-        forget();
     }
     const int kOut = MEDYAN_FF_COUNT + 1;
     // a force contribution out of the fixed-point range (bit 2) leaves the

@@ -996,7 +996,8 @@ CGState batch_start_state(const medyan_cg_params* p, int nb) {
 }
 
 // Batched CGMethod::minimize over the packed replicas; see the kernels above.
-medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p) {
+medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p,
+                           const std::vector<PackedCarry>& carry) {
     const int R = pb.R;
     if (!p || p->method < 0 || p->method > 2 || !(p->max_dist > 0) || !(p->lambda_max > 0) || p->line_search < 0 ||
         p->line_search > 1)
@@ -1035,11 +1036,31 @@ medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p)
     if (e != cudaSuccess) return cuda_status(e);
 
     // energiesBefore, then the first force, F.F, d = F
-    k_b_act_all<<<(R + 255) / 256, 256, 0, s>>>(R, pb.act.raw());
-    b_energy_pass(pb, nullptr, pb.Lzero.raw(), s);
-    k_b_decide<<<1, 1, 0, s>>>(0, pb.st.raw(), pb.Lr.raw(), pb.out.raw(), pb.off.raw(), pb.es.fb_count, pb.es.bad);
-    k_b_record<<<(R + 127) / 128, 128, 0, s>>>(R, pb.st.raw(), pb.out.raw(), pb.eout.raw(), 1);
-    b_step(pb, prec, s);
+    if ((int)carry.size() < R) {
+        k_b_act_all<<<(R + 255) / 256, 256, 0, s>>>(R, pb.act.raw());
+        b_energy_pass(pb, nullptr, pb.Lzero.raw(), s);
+        k_b_decide<<<1, 1, 0, s>>>(0, pb.st.raw(), pb.Lr.raw(), pb.out.raw(), pb.off.raw(), pb.es.fb_count, pb.es.bad);
+        k_b_record<<<(R + 127) / 128, 128, 0, s>>>(R, pb.st.raw(), pb.out.raw(), pb.eout.raw(), 1);
+        b_step(pb, prec, s);
+    }
+    // then, in place of what that gave them, the replicas that stand further on
+    for (const PackedCarry& c : carry) {
+        const size_t o = 3 * (size_t)pb.base[c.r], n = sizeof(double) * 3 * (size_t)(pb.base[c.r + 1] - pb.base[c.r]);
+        auto put = [&](void* to, const void* from, size_t bytes, cudaMemcpyKind kind) {
+            if (e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, kind, s);
+        };
+        CGState st = c.st;
+        st.full_passes = 1;
+        put(pb.st.raw() + c.r, &st, sizeof st, cudaMemcpyHostToDevice);
+        put(pb.x.raw() + o, c.x, n, cudaMemcpyDeviceToDevice);
+        put(pb.d.raw() + o, c.d, n, cudaMemcpyDeviceToDevice);
+        put(pb.fcur.raw() + o, c.f, n, cudaMemcpyDeviceToDevice);
+        put(pb.minE.raw() + o, c.min_e, n, cudaMemcpyDeviceToDevice);
+        put(pb.Lr.raw() + c.r, c.lam, sizeof(LambdaSet), cudaMemcpyDeviceToDevice);
+        put(pb.eout.raw() + (size_t)c.r * 2 * kOut, c.eout, sizeof(double) * 2 * kOut, cudaMemcpyDeviceToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // st leaves
+        if (e != cudaSuccess) return cuda_status(e);
+    }
 
     if (pb.graph && (pb.graph_gen != pb.gen || pb.graph_prec != prec || pb.graph_det != pb.deterministic)) {
         cudaGraphExecDestroy(pb.graph);

@@ -310,6 +310,12 @@ bool batch_loop_takes(const std::vector<medyan_mech*>& h) {
     return true;
 }
 
+PackedCarry batch_loop_carry(const PackedBatch& pb, int r, const CGState& st, int to) {
+    const size_t o = 3 * (size_t)pb.lbase[r];
+    return PackedCarry{to, st, pb.lx.raw() + o, pb.ld.raw() + o, (st.parity ? pb.lf1 : pb.lf0).raw() + o,
+                       pb.lmin.raw() + o, pb.llam.raw() + r, pb.leout.raw() + (size_t)r * 2 * (MEDYAN_FF_COUNT + 1)};
+}
+
 medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h, const medyan_cg_params* p,
                              double* const* coords, double* const* forces, CGState* st, double* eout, int* outcome,
                              int* force_status) {
@@ -429,8 +435,8 @@ medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h
     *force_status = pw[(size_t)R * kLoopWords + 1];
     for (int r = 0; r < R; ++r) {
         outcome[r] = pw[(size_t)r * kLoopWords + 2];
+        if (outcome[r] == kLoopDone || outcome[r] == kLoopHandOver) st[r] = ps[r];
         if (outcome[r] != kLoopDone) continue;
-        st[r] = ps[r];
         std::memcpy(eout + (size_t)r * kE, pe + (size_t)r * kE, sizeof(double) * kE);
         for (int out = 0; out < 2; ++out) {
             double* to = out == 0 ? coords[r] : (forces ? forces[r] : nullptr);

@@ -106,16 +106,29 @@ medyan_status batch_streams(PackedBatch& pb);
 // minimization there: coordinates in and out of the callers' arrays, the state
 // and energies of replica r into st[r] and eout + 2 r (MEDYAN_FF_COUNT + 1).
 // outcome[r] is not kLoopDone for a replica that met a pair which needs a
-// quadrature: nothing of it is written.
+// quadrature: nothing of it is written but, at kLoopHandOver, the state that the
+// packed run goes on from.
 bool batch_loop_takes(const std::vector<medyan_mech*>& h);
 medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h, const medyan_cg_params* p,
                              double* const* coords, double* const* forces, CGState* st, double* eout, int* outcome,
                              int* force_status);
 // The start state of a replica with nb beads.
 CGState batch_start_state(const medyan_cg_params* p, int nb);
+// A minimization in progress (the resident loop's) that a packed run goes on with.
+struct PackedCarry {
+    int r;                            // its replica in the packing
+    CGState st;
+    const double *x, *d, *f, *min_e;  // on the device, the replica's beads
+    const LambdaSet* lam;             // step sizes of the pending pass
+    const double* eout;
+};
+// Its replica r of pb's last resident run, for replica `to` of a packing.
+PackedCarry batch_loop_carry(const PackedBatch& pb, int r, const CGState& st, int to);
 // Runs one batched minimization on the packed arrays (coordinates already in
-// pb.x); results stay on the device (pb.x, pb.fcur, pb.st, pb.eout).
-medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p);
+// pb.x), of the replicas in carry from where they stand; results stay on the
+// device (pb.x, pb.fcur, pb.st, pb.eout).
+medyan_status cg_batch_run(PackedBatch& pb, int prec, const medyan_cg_params* p,
+                           const std::vector<PackedCarry>& carry = {});
 // Mean time (ms) of one packed evaluate (energy and forces of every replica
 // at pb.x) after two warm-up passes; for the autotuner.
 medyan_status cg_batch_time_evaluate(PackedBatch& pb, int prec, int reps, float* ms);
