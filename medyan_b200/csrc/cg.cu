@@ -720,6 +720,7 @@ static LoopArgs loop_args(medyan_mech* h, const CGLaunch& c) {
     a.f0 = c.f0;
     a.f1 = c.f1;
     a.min_e = c.minE;
+    a.lo = h->cg_lo.raw();  // used by the 256-thread blocks' floating-point sums
     a.st = c.st;
     a.lam = c.L;
     a.eout = h->cg_eout.raw();
@@ -755,12 +756,15 @@ medyan_status cg_enqueue(medyan_mech* h, const medyan_cg_params* p, const double
     if (e == cudaSuccess && h->cg_team > 0)
         e = h->cg_rows.reserve(loop_erow_doubles(loop_row_count(h->chain, h->ff)) + loop_vrow_doubles(vec_blocks(n3)));
     if (e == cudaSuccess && h->cg_team > 0) e = h->cg_words.reserve(kLoopWords);
+    const bool parts = h->cg_team > 0 && !h->deterministic && h->n_beads <= kLoopWideBeads;
+    if (e == cudaSuccess && parts) e = h->cg_lo.reserve(n3);
     if (e != cudaSuccess) return cuda_status(e);
     const CGLaunch c = make_launch(h);
     e = staged(h, coord_in, kStageMinimize) ? staged_in(h, coord_in, c.x) : coords_to_device(h, coord_in, c.x, s);
     if (e == cudaSuccess) e = cg_start(h, c, s);
     if (e == cudaSuccess && h->cg_team > 0) {
         e = cudaMemsetAsync(h->cg_words.raw(), 0, sizeof(int) * kLoopWords, s);
+        if (e == cudaSuccess && parts) e = cudaMemsetAsync(h->cg_lo.raw(), 0, sizeof(double) * n3, s);
         if (e == cudaSuccess) e = launch_cg_loop(loop_args(h, c), h->prec, h->cg_team, s);
     } else if (e == cudaSuccess) {
         e = cg_graph_run(h, c, s);

@@ -16,6 +16,7 @@ struct LoopArgs {
     int vb;            // blocks of the vector passes' summation order (vec_blocks, or 1)
     int fixed;         // deterministic force sums
     double *x, *d, *f0, *f1, *min_e;
+    double* lo;        // low parts of the force sums, zero at the launch (floating-point sums in two parts only)
     CGState* st;       // parameters in, final state out
     LambdaSet* lam;    // pending step sizes when the loop hands over
     double* eout;      // [2][MEDYAN_FF_COUNT + 1]: energies before and after

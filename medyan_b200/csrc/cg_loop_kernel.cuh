@@ -165,18 +165,44 @@ struct Pos {
     }
 };
 
+// Floating-point sums in two parts: v's multiple of 2^-26 is added to the force, the rest to lo.
+// The first sums are exact (below 2^27), whatever the order in which the team's
+// blocks add; the second vary by rounding of parts below 2^-27, 1e-24 pN. Added
+// as they are, a bead's three or more contributions gave other last bits from run to
+// run, and a minimization by chance reaches its tolerance on another path: of 400
+// minimizations of 12 filaments of 6 cylinders 31 to 41 ended far from the oracle's
+// energy; now none, all alike. It costs 3 to 6 % of a minimization (550 beads 852 and 908
+// us, 10,500 897 and 970, 52,500 1,970 and 2,085, a batch of 128 replicas 6.8 and 7.1 ms),
+// at 100,800 beads 13 %, and larger networks' sums differ from run to run in every
+// form: the 512-thread blocks of a single network add as it is (kParts).
+template <bool BATCH>
+constexpr bool kParts = BATCH || kLoopThreads == 256;
+constexpr double kHiCenter = 1.5 * 67108864.0, kHiRange = 33554432.0;
+__device__ __forceinline__ void add_parts(double* f, double* lo, double v) {
+    const bool in = fabs(v) < kHiRange;  // else as it is (NaN and infinities too)
+    const double h = in ? __dadd_rn(__dadd_rn(v, kHiCenter), -kHiCenter) : v;
+    const double l = in ? v - h : 0.0;
+    red_add(f, h);
+    if (l != 0.0) red_add(lo, l);
+}
+
 // Force target with the kind of sums fixed at compile time: half the code of
 // every addition, in a kernel that is bound by fetching its instructions.
-template <bool FIXED>
+template <bool FIXED, bool PARTS>
 struct Sink {
     int* status;
+    double* lo;
 };
-template <bool FIXED, class R>
-__device__ __forceinline__ void target_add(const Sink<FIXED>& t, double* f, int off, R fx, R fy, R fz) {
+template <bool FIXED, bool PARTS, class R>
+__device__ __forceinline__ void target_add(const Sink<FIXED, PARTS>& t, double* f, int off, R fx, R fy, R fz) {
     if constexpr (FIXED) {
         red_add_fixed(f + off, fixed_of(double(fx), t.status));
         red_add_fixed(f + off + 1, fixed_of(double(fy), t.status));
         red_add_fixed(f + off + 2, fixed_of(double(fz), t.status));
+    } else if constexpr (PARTS) {
+        add_parts(f + off, t.lo + off, double(fx));
+        add_parts(f + off + 1, t.lo + off + 1, double(fy));
+        add_parts(f + off + 2, t.lo + off + 2, double(fz));
     } else {
         add_force(f, off, fx, fy, fz);
     }
@@ -242,14 +268,14 @@ __device__ __forceinline__ double tree8(const double (*v)[kRowVals], int j) {
 // pass: the kernel's code is several times an SM's instruction cache, and with
 // kinds dealt round the blocks a task spent half its time fetching
 // instructions (a pass of 2000 filaments of 20 cylinders 13.2 against 11.9 us).
-template <class R, bool FIXED>
+template <class R, bool FIXED, bool PARTS>
 __device__ __noinline__ void pass(Pos P, int K, bool force, double lam_f, double* f, int* status, int parity) {
     Smem& sm = smem();
     const LoopArgs& a = sm.a;
     const Team& tm = sm.tm;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane & 3;
     const DeviceFF& ff = a.ff;
-    const Sink<FIXED> t{status};
+    const Sink<FIXED, PARTS> t{status, a.lo};
     bool bad = false;
     int f_blocks = 0;  // blocks that the force tasks fill
     // The pairs' forces, the longest tasks, take four warps of a block, one per
@@ -624,6 +650,7 @@ __device__ void minimize() {
     const LoopArgs& a = sm.a;
     const Team& tm = sm.tm;
     CGState& s = sm.s;
+    constexpr bool PARTS = !FIXED && kParts<BATCH>;
     auto words = [](auto& v) { return reinterpret_cast<int*>(&v); };
     for (int i = threadIdx.x; i < (int)(sizeof(CGState) / 4); i += kLoopThreads) words(s)[i] = words(*a.st)[i];
     if (threadIdx.x == 0) {
@@ -699,7 +726,7 @@ __device__ void minimize() {
     const Pos at_x{a.x, nullptr, nullptr, 0.0, 0.0, false};
 
     // energies before, and the first force
-    pass<R, FIXED>(at_x, 1, true, 0.0, other(), a.status, parity);
+    pass<R, FIXED, PARTS>(at_x, 1, true, 0.0, other(), a.status, parity);
     if (!team_sync()) return leave(kLoopLost);
     if (!add_rows<BATCH>(1, parity)) return leave(kLoopRestart);
     parity ^= 1;
@@ -714,12 +741,12 @@ __device__ void minimize() {
             double *Fn = other(), *Fc = current();
             const double lam = s.lam_move, beta = sm.beta;
             const bool copy = sm.min_pending;
-            double *x = a.x, *d = a.d, *min_e = a.min_e;
+            double *x = a.x, *d = a.d, *min_e = a.min_e, *lo = a.lo;
             struct In {
-                double x, d, fn, fc;
+                double x, d, fn, fc, lo;
             };
             vector_pass(
-                a.vrow, [&](int i) { return In{x[i], d[i], Fn[i], Fc[i]}; },
+                a.vrow, [&](int i) { return In{x[i], d[i], Fn[i], Fc[i], PARTS ? lo[i] : 0.0}; },
                 [&](int i, In v, Sums& q) {
                     const double dn = v.fc + beta * v.d;  // shiftSearchDir (CGMethod.cpp:356-360)
                     if (copy) min_e[i] = v.x;
@@ -727,6 +754,10 @@ __device__ void minimize() {
                     x[i] = move1(v.x, lam, dn);
                     if constexpr (FIXED) {
                         v.fn = double(__double_as_longlong(v.fn)) / kFixedScale;
+                        Fn[i] = v.fn;
+                    } else if constexpr (PARTS) {
+                        v.fn += v.lo;
+                        lo[i] = 0.0;
                         Fn[i] = v.fn;
                     }
                     Fc[i] = 0.0;
@@ -760,7 +791,10 @@ __device__ void minimize() {
             const double* F = current();
             const double beta = s.dir_mode ? 0.0 : s.beta;
             if (!moved)
-                for (int i = first; i < a.n3; i += step) other()[i] = 0.0;
+                for (int i = first; i < a.n3; i += step) {
+                    other()[i] = 0.0;
+                    if constexpr (PARTS) a.lo[i] = 0.0;
+                }
             struct In {
                 double f, d;
             };
@@ -794,7 +828,7 @@ __device__ void minimize() {
         while (s.ls_active && !s.done) {
             const int K = s.ls_immediate_fail ? 0 : sm.L.K;
             if (K > 0) {
-                pass<R, FIXED>(along, K, sm.spec_on, s.spec_lam, other(), &a.st->spec_status, parity);
+                pass<R, FIXED, PARTS>(along, K, sm.spec_on, s.spec_lam, other(), &a.st->spec_status, parity);
                 if (!team_sync()) return leave(kLoopLost);
                 if (!add_rows<BATCH>(K, parity)) return leave(kLoopHandOver);
                 parity ^= 1;
@@ -816,10 +850,13 @@ __device__ void minimize() {
         if (!s.done && !s.skip_force && !sm.hit) {
             double* F = other();
             if (sm.dirty) {
-                for (int i = first; i < a.n3; i += step) F[i] = 0.0;
+                for (int i = first; i < a.n3; i += step) {
+                    F[i] = 0.0;
+                    if constexpr (PARTS) a.lo[i] = 0.0;
+                }
                 if (!team_sync()) return leave(kLoopLost);
             }
-            pass<R, FIXED>(along, 0, true, s.lam_move, F, a.status, parity);
+            pass<R, FIXED, PARTS>(along, 0, true, s.lam_move, F, a.status, parity);
             if (!team_sync()) return leave(kLoopLost);
             if (!add_rows<BATCH>(0, parity)) return leave(kLoopHandOver);
             parity ^= 1;
@@ -844,7 +881,7 @@ __device__ void minimize() {
     // network's energy buffer holds those of its coordinates all the same
     const bool failed = s.status == MEDYAN_ERR_LINE_SEARCH;
     if (!failed || a.e_last) {
-        pass<R, FIXED>(at_x, 1, false, 0.0, nullptr, nullptr, parity);
+        pass<R, FIXED, PARTS>(at_x, 1, false, 0.0, nullptr, nullptr, parity);
         if (!team_sync()) return leave(kLoopLost);
         if (!add_rows<BATCH>(1, parity)) return leave(kLoopHandOver);
         if (a.e_last && tm.rank == 0 && threadIdx.x < kOut) a.e_last[threadIdx.x] = sm.out[threadIdx.x];

@@ -232,7 +232,7 @@ struct medyan_mech {
     mb::DevBuf<mb::LambdaSet> cg_lam;
     // resident loop (cg_loop_kernel.cuh): partial rows, control words; the team of the
     // minimization in flight (0: the graph loop)
-    mb::DevBuf<double> cg_rows;
+    mb::DevBuf<double> cg_rows, cg_lo;
     mb::DevBuf<int> cg_words;
     int cg_team = 0;
     mb::LoopRoom loop_room;

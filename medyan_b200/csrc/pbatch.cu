@@ -351,6 +351,7 @@ medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h
         }
         const size_t n3 = 3 * (size_t)pb.lbase[R];
         for (DevBuf<double>* b : {&pb.lx, &pb.ld, &pb.lf0, &pb.lf1, &pb.lmin}) res(*b, n3);
+        res(pb.llo, pb.deterministic ? 0 : n3);
         res(pb.leout, (size_t)R * kE);
         res(pb.lst, R);
         res(pb.llam, R);
@@ -372,6 +373,7 @@ medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h
             a.f0 = pb.lf0.raw() + o;
             a.f1 = pb.lf1.raw() + o;
             a.min_e = pb.lmin.raw() + o;
+            a.lo = pb.deterministic ? nullptr : pb.llo.raw() + o;
             a.st = pb.lst.raw() + r;
             a.lam = pb.llam.raw() + r;
             a.eout = pb.leout.raw() + (size_t)r * kE;
@@ -417,6 +419,7 @@ medyan_status batch_loop_run(PackedBatch& pb, const std::vector<medyan_mech*>& h
     if (e == cudaSuccess) e = cudaMemcpyAsync(pb.lst.raw(), ps, sizeof(CGState) * R, cudaMemcpyHostToDevice, s);
     for (DevBuf<double>* b : {&pb.ld, &pb.lf0, &pb.lf1})
         if (e == cudaSuccess) e = cudaMemsetAsync(b->raw(), 0, bytes, s);
+    if (e == cudaSuccess && !pb.deterministic) e = cudaMemsetAsync(pb.llo.raw(), 0, bytes, s);
     if (e == cudaSuccess)
         e = cudaMemsetAsync(pb.loop_words.raw(), 0, sizeof(int) * (size_t)(R + 1) * kLoopWords, s);
     if (e == cudaSuccess)

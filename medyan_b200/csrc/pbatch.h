@@ -78,7 +78,7 @@ struct PackedBatch {
     // order of the queue, pinned staging of coordinates and forces
     DevBuf<LoopArgs> loop_args;
     DevBuf<int> loop_words, loop_order;
-    DevBuf<double> loop_rows, lx, ld, lf0, lf1, lmin, leout;
+    DevBuf<double> loop_rows, lx, ld, lf0, lf1, lmin, llo, leout;
     DevBuf<CGState> lst;
     DevBuf<LambdaSet> llam;
     std::vector<int> lbase;           // bead base of each replica (R + 1)
