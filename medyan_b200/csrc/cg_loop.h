@@ -37,8 +37,15 @@ constexpr int kLoopDone = 0, kLoopHandOver = 1, kLoopRestart = 2, kLoopLost = 3;
 
 constexpr int kLoopCluster = 16;    // teams of up to this many blocks are thread-block clusters
 constexpr int kLoopGrid = 148;      // blocks of the largest team, a cooperative grid (one block per SM)
-constexpr int kLoopBeads = 350000;  // larger networks run in the graph loop
-constexpr int kLoopWideBeads = 75000;  // larger ones take blocks of 512 threads
+// Larger networks run in the graph loop. Microseconds of an iteration, resident and
+// graph loop, FP64 with fixed-point sums: 25,200 beads 22 and 54, 100,800 47 and 77,
+// 201,600 57 and 73, 235,200 61 and 75, 302,400 70 and 79, 348,600 80-103 and 74-90,
+// 420,000 91 and 97 (with atomic sums 84 and 78). Whole calls with 40 energy calls,
+// resident and graph: 302,400 5.4-5.7 and 5.5-5.7 ms, 348,600 6.2-6.5 and 6.1.
+constexpr int kLoopBeads = 310000;
+// Larger ones take blocks of 512 threads. 256 and 512: 25,200 beads 21.7 and 22.7 us,
+// 52,500 27.7 and 30.7, 76,440 39.1 and 37.0, 100,800 55 and 47, 201,600 63 and 57.
+constexpr int kLoopWideBeads = 75000;
 
 // Blocks of a team for this network, 0 when the network is better off in the
 // graph loop, or the device has no room for the team.
@@ -60,7 +67,10 @@ cudaError_t launch_cg_loop_wide(const LoopArgs& a, int prec, int team, cudaStrea
 // The replicas of a batch (arguments on the device; vb = 1, the order of the
 // packed batch's sums), taken in the order given, each by one cluster. bounded:
 // a call limit bounds the iterations.
-constexpr int kLoopBatchBeads = 20000;  // larger replicas run in the packed batch
+// Larger replicas run in the packed batch. 16 replicas over 100 energy calls, resident
+// and packed: 10,500 beads each 11.4 and 14.1 ms, 18,900 21.3 and 25.0. The line lies
+// below where the two meet: 8 replicas of 25,200 16.3 and 21.8, of 63,000 41 and 76.
+constexpr int kLoopBatchBeads = 20000;
 cudaError_t launch_cg_loop_batch(const LoopArgs* replicas, const int* order, int n, int* queue, int prec, bool fixed,
                                  bool bounded, cudaStream_t s);
 

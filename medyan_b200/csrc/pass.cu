@@ -103,7 +103,12 @@ constexpr int main_blocks_per_sm() {
     return kMainBlocksPerSM;
 }
 constexpr int kExclThreadsMax = 128;
-constexpr int kQuadPairs = 8000;  // pairs up to which four lanes share one (pass_geometry)
+// Pairs up to which four lanes share one (pass_geometry). Four lanes and one, us of a
+// pass, FP64: forces 1,671 pairs 10.3 and 12.3, 4,481 10.3 and 12.3, 6,623 12.3 and
+// 12.3; evaluate 1,671 pairs 14.5 and 16.1, 3,005 17.3 and 16.7, 6,623 18.5 and 17.6,
+// 9,795 21.5 and 19.9, 23,114 28.4 and 25.0. The line stands where the forces, the
+// minimizer's and the larger gain, no longer differ.
+constexpr int kQuadPairs = 8000;
 
 // Positions of a pass: x, or x + lam*d rounded as calcCoordLineSearch.
 struct Pos {
