@@ -702,7 +702,8 @@ def batch_extras(n_replicas: int = 256) -> dict:
                      "second_run_identical": identical,
                      "one_at_a_time_minimizations_per_s": m / seq, "iterations_mean": float(np.mean(its)),
                      "iterations_max": int(max(its)), "statuses": sorted(set(int(v) for v in st)),
-                     "launch_shapes": shapes,
+                     # of packed passes; the minimizations above run in the resident loop
+                     "packed_launch_shapes": shapes,
                      "atomic_sums": {"seconds": dta, "minimizations_per_s": n_replicas / dta,
                                      "iterations_mean": float(np.mean(itsa)), "iterations_max": int(max(itsa))}}
     return out
