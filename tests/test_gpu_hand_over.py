@@ -73,6 +73,21 @@ def test_handed_over_is_the_graph_loop(gpu_lib, oracle, size, line_search, preci
         assert np.abs(xo - want[1]).max() <= (1e-7 if line_search == "BACKTRACKING" else 1e-6)
 
 
+@pytest.mark.parametrize("size", [(4, 3, 700.0), (60, 10, 1800.0)])
+def test_floating_sums_are_handed_over(gpu_lib, oracle, size):
+    """The same with floating-point force sums, which the loop keeps in two parts."""
+    sv, x = system(*size)
+    so, xo, fo, ro = oracle.minimize(sv, x, params())
+    with ForceFieldManager("fp64") as ff:
+        ff.vectorize_all_force_fields(sv)
+        s, xg, f, r = ff.minimize(x, params())
+    with BatchMinimizer([sv, sv], "fp64") as b:
+        sb, xb, fb, rb = b.minimize([x, x], params())
+    for got in ((s, xg, f, r), (sb[1], xb[1], fb[1], rb[1])):
+        assert got[0] == so == 0 and counts(got[3]) == counts(ro)
+        assert np.abs(got[1] - xo).max() <= 1e-7 and np.abs(got[2] - fo).max() <= 1e-7 * max(np.abs(fo).max(), 1.0)
+
+
 @pytest.mark.parametrize("line_search", ["BACKTRACKING", "QUADRATIC"])
 @pytest.mark.parametrize("turning", [(2,), (0, 3), (0, 1, 2, 3, 4)])
 def test_batch_hands_over_some_replicas(gpu_lib, line_search, turning):
